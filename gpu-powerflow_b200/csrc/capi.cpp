@@ -119,8 +119,11 @@ bool copy_plan_array(const Engine& e, const char* name, int32_t* out, int64_t ca
   CUPF_ARR("diag22", ja.diag22)
 #undef CUPF_ARR
   if (n == "factor_level_warps" || n == "backward_launch_warps" || n == "factor_level_tiers" ||
-      n == "tc_threshold" || n == "factor_level_placement") {  // the autotuner's choices, each launch's kernel
-    const std::vector<int32_t> w = n == "factor_level_warps"       ? e.factor_level_warps()
+      n == "tc_threshold" || n == "factor_level_placement" ||  // the autotuner's choices, each launch's kernel
+      n.compare(0, 9, "task_meta") == 0 || n.compare(0, 10, "task_words") == 0 ||
+      n.compare(0, 11, "task_stages") == 0 || n.compare(0, 11, "task_sweep_") == 0) {
+    const std::vector<int32_t> w = n.compare(0, 5, "task_") == 0  ? e.task_array(n)
+                                   : n == "factor_level_warps"    ? e.factor_level_warps()
                                    : n == "factor_level_tiers"     ? e.factor_level_tiers()
                                    : n == "factor_level_placement" ? e.factor_level_placements()
                                    : n == "tc_threshold"           ? std::vector<int32_t>{e.tc_threshold()}

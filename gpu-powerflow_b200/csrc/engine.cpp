@@ -18,11 +18,14 @@
 #include <cstdlib>
 #include <cstring>
 #include <limits>
+#include <map>
+#include <memory>
 #include <stdexcept>
 #include <string>
 
 #include "kernels.hpp"
 #include "static_scratch.hpp"
+#include "task_plan.hpp"
 
 namespace cupf_b200 {
 
@@ -92,6 +95,18 @@ std::vector<long long> to_ll(const std::vector<T>& v) {
 
 }  // namespace
 
+// Subtree tasks of the factorization and the sweeps (task_plan.hpp), one set
+// per class of batch size, and the level launches of the fronts no
+// factorization task covers, with launch records and source lists of their
+// own.
+struct Engine::TaskSet {
+  TaskPlan tasks;
+  SweepPlan sweeps;  // empty: a front is too large, and the sweeps run level by level
+  DBuf task_meta, task_words, sweep_meta, sweep_words, rest_meta, rest_src, rest_dst;
+  std::vector<LevelLaunch> rest;
+  bool uploaded = false;
+};
+
 struct Engine::Impl {
   // grid
   DBuf y_ptr, y_col, y_row, y_diag, y_re, y_im, map11, map21, map12, map22, bus_fa, bus_fm, bus_fa_p, bus_fm_p, pv, pq,
@@ -100,6 +115,10 @@ struct Engine::Impl {
   DBuf fsz, nc, first, front_ptr, front_rows, u_off, l_off, cb_off, tv_off, arow_ptr, arow_q, arow_col, crow_ptr,
       crow_child, crow_r, crow_src, crow_dst, asm_ptr, asm_local, perm, iperm, row_iperm, col_perm, level_fronts, fe_split, fe_dst, fe_src, front_meta;
   std::vector<LevelLaunch> levels;
+  std::map<int, std::unique_ptr<TaskSet>> task_sets;
+  TaskSet* ts = nullptr;  // of the current batch
+  int graph_lanes = 0;    // tasks' scenarios of the captured solve
+  int task_lanes() const { return B == 1 ? 1 : Bp; }  // scenarios the tasks cover (padding included)
   // backward sweep: the narrow top levels (launch-list entries from bw_first
   // on) run as one launch over bw_bounds (descending level boundaries)
   int bw_first = 0, bw_nlev = 0;
@@ -214,6 +233,14 @@ bool Engine::tf32_factors() const { return cfg_.factor_precision == kFactorTF32 
 
 bool Engine::single_system() const { return cfg_.batch1_schedule == 0 && d_->B == 1; }
 
+bool Engine::use_tasks() const {
+  if (d_->ts->tasks.stages.empty() || (d_->B == 1 && cfg_.batch1_schedule == 1)) return false;
+  // a single small system: one tree launch costs less than a launch per stage
+  // (118 buses, 94 fronts: 464 against 500 us per graph-mode solve; 2,000
+  // buses, 1,671 fronts: 1,265 against 1,125 us)
+  return !single_system() || (d_->ts->rest.empty() && fp_.P >= 256);
+}
+
 // The single-system factorization as one tree launch: batch 1, no
 // tensor-core launch among the levels, every front and list in shared memory.
 bool Engine::single_tree(size_t elem_bytes) const {
@@ -226,10 +253,14 @@ bool Engine::single_tree(size_t elem_bytes) const {
 void Engine::assign_tiers(int tc_min) {
   const int wide_min = std::min(cfg_.wide_min_front > 0 ? cfg_.wide_min_front : kWideFrontRows, kWideFrontRows);
   tc_min_ = tf32_factors() ? tc_min : 0;
-  for (auto& lv : d_->levels) {
-    lv.tier = lv.max_fsz >= wide_min ? 1 : 0;
-    if (tc_min_ > 0 && lv.max_fsz >= tc_min_) lv.tier = 2;
-  }
+  std::vector<std::vector<LevelLaunch>*> sets{&d_->levels};
+  for (auto& s : d_->task_sets)
+    if (s.second) sets.push_back(&s.second->rest);
+  for (auto* levels : sets)
+    for (auto& lv : *levels) {
+      lv.tier = lv.max_fsz >= wide_min ? 1 : 0;
+      if (tc_min_ > 0 && lv.max_fsz >= tc_min_) lv.tier = 2;
+    }
 }
 
 std::vector<int32_t> Engine::factor_level_tiers() const {
@@ -349,6 +380,124 @@ void Engine::update_ybus_values(const double* ydata) {
   adjoint_ready_ = false;
 }
 
+// The level launches of the fronts given level by level.
+std::vector<LevelLaunch> Engine::level_launches(const std::vector<std::vector<int32_t>>& by_level) const {
+  std::vector<LevelLaunch> out;
+  auto bucket = [](int32_t f) {
+    for (int32_t c : {6, 8, 10, 12, 16, 20, 24, 32, 48, 64})
+      if (f <= c) return c;
+    return 1 << 30;
+  };
+  constexpr size_t kMinRun = 64;
+  int32_t begin = 0;
+  for (const auto& lf : by_level) {
+    if (lf.empty()) continue;
+    std::vector<size_t> cuts{0};
+    for (size_t q = 1; q < lf.size(); ++q) {
+      if (bucket(fp_.fsz[lf[q]]) == bucket(fp_.fsz[lf[q - 1]])) continue;
+      if (q - cuts.back() >= kMinRun && lf.size() - q >= kMinRun) cuts.push_back(q);
+    }
+    cuts.push_back(lf.size());
+    for (size_t c = 0; c + 1 < cuts.size(); ++c) {
+      LevelLaunch lv;
+      lv.begin = begin + (int32_t)cuts[c];
+      lv.count = (int32_t)(cuts[c + 1] - cuts[c]);
+      for (size_t q = cuts[c]; q < cuts[c + 1]; ++q) {
+        const int32_t f = lf[q];
+        lv.max_fsz = std::max(lv.max_fsz, fp_.fsz[f]);
+        lv.max_nc = std::max(lv.max_nc, fp_.nc[f]);
+        lv.max_src = std::max<int>(lv.max_src, (int)(fp_.fe_ptr[f + 1] - fp_.fe_ptr[f]));
+      }
+      out.push_back(lv);
+    }
+    begin += (int32_t)lf.size();
+  }
+  return out;
+}
+
+// Cuts the front tree into subtree tasks for the batch class.  Fronts that an
+// option sends to another kernel (the any-size tier, the tensor cores) stay
+// with the level launches of the factorization, as do fronts too large for a
+// task.
+Engine::TaskSet& Engine::task_set(int cls) const {
+  auto& d = *d_;
+  auto& slot = d.task_sets[cls];
+  if (slot) return *slot;
+  slot = std::make_unique<TaskSet>();
+  int limit = std::min(cfg_.wide_min_front > 0 ? cfg_.wide_min_front : kWideFrontRows, kWideFrontRows);
+  if (tf32_factors())
+    limit = std::min(limit, cfg_.tc_min_front > 0 ? cfg_.tc_min_front
+                            : cfg_.autotune       ? kTcSmallestMinFront
+                                                  : kTcDefaultMinFront);
+  slot->tasks = build_task_plan(fp_, limit, factor_task_specs(cls, factor_is_double() ? 8 : 4));
+  std::vector<std::vector<int32_t>> by_level(fp_.num_levels);
+  for (int32_t L = 0; L < fp_.num_levels; ++L)
+    by_level[L].assign(fp_.level_fronts.begin() + fp_.level_ptr[L], fp_.level_fronts.begin() + fp_.level_ptr[L + 1]);
+  std::vector<int32_t> counts(fp_.P, 0);
+  for (const LevelLaunch& lv : level_launches(by_level))
+    for (int32_t q = lv.begin; q < lv.begin + lv.count; ++q) counts[fp_.level_fronts[q]] = lv.count;
+  slot->sweeps = build_sweep_plan(fp_, sweep_task_specs(cls), counts);
+  return *slot;
+}
+
+// Makes the current batch's task set the one in use (uploading it at its
+// first batch).
+void Engine::select_tasks() {
+  auto& d = *d_;
+  TaskSet& ts = task_set(task_class(fp_.P, d.B));
+  d.ts = &ts;
+  if (ts.uploaded) return;
+  ts.task_meta.upload(ts.tasks.meta);
+  ts.task_words.upload(ts.tasks.words);
+  ts.sweep_meta.upload(ts.sweeps.meta);
+  ts.sweep_words.upload(ts.sweeps.words);
+  if (!ts.tasks.stages.empty()) {
+    // the fronts no task covers, level by level
+    std::vector<std::vector<int32_t>> by_level(fp_.num_levels);
+    std::vector<int32_t> order, qof(fp_.P), meta;
+    for (int32_t L = 0; L < fp_.num_levels; ++L)
+      for (int32_t q = fp_.level_ptr[L]; q < fp_.level_ptr[L + 1]; ++q) {
+        const int32_t p = fp_.level_fronts[q];
+        qof[p] = q;
+        if (!ts.tasks.covered[p]) by_level[L].push_back(p);
+      }
+    ts.rest = level_launches(by_level);
+    for (const auto& lv : by_level) order.insert(order.end(), lv.begin(), lv.end());
+    for (int32_t p : order)
+      meta.insert(meta.end(), fp_.front_meta.begin() + (size_t)qof[p] * kFrontMetaInts,
+                  fp_.front_meta.begin() + (size_t)(qof[p] + 1) * kFrontMetaInts);
+    ts.rest_meta.upload(meta);
+    pad_lists(ts.rest, order, ts.rest_src, ts.rest_dst);
+    assign_tiers(tc_min_);
+  }
+  ts.uploaded = true;
+}
+
+// Source lists in launch order, each padded to its launch's longest.
+template <typename Buf>
+void Engine::pad_lists(std::vector<LevelLaunch>& levels, const std::vector<int32_t>& order, Buf& src, Buf& dst) const {
+  std::vector<long long> psrc;
+  std::vector<int32_t> pdst;
+  for (auto& lv : levels) {
+    lv.max_src = std::max(lv.max_src, 1);
+    lv.fe_base = (long long)psrc.size();
+    for (int32_t q = lv.begin; q < lv.begin + lv.count; ++q) {
+      const int32_t f = order[q];
+      const int64_t a = fp_.fe_ptr[f], z = fp_.fe_ptr[f + 1];
+      for (int64_t e = a; e < z; ++e) {
+        psrc.push_back(fp_.fe_src[e]);
+        pdst.push_back(fp_.fe_dst[e]);
+      }
+      for (int64_t e = z - a; e < lv.max_src; ++e) {
+        psrc.push_back(0);
+        pdst.push_back(-1);
+      }
+    }
+  }
+  src.upload(psrc);
+  dst.upload(pdst);
+}
+
 void Engine::upload_plan() {
   auto& d = *d_;
   d.fsz.upload(fp_.fsz);
@@ -400,34 +549,12 @@ void Engine::upload_plan() {
   // size (fronts are size-sorted inside a level) when both sides of a cut
   // hold enough fronts to fill the GPU, so that the shared memory of a launch
   // is sized for its own fronts rather than the level's largest.
-  d.levels.clear();
-  auto bucket = [](int32_t f) {
-    for (int32_t c : {6, 8, 10, 12, 16, 20, 24, 32, 48, 64})
-      if (f <= c) return c;
-    return 1 << 30;
-  };
-  constexpr int32_t kMinRun = 64;
-  for (int32_t L = 0; L < fp_.num_levels; ++L) {
-    const int32_t b0 = fp_.level_ptr[L], b1 = fp_.level_ptr[L + 1];
-    std::vector<int32_t> cuts{b0};
-    for (int32_t q = b0 + 1; q < b1; ++q) {
-      if (bucket(fp_.fsz[fp_.level_fronts[q]]) == bucket(fp_.fsz[fp_.level_fronts[q - 1]])) continue;
-      if (q - cuts.back() >= kMinRun && b1 - q >= kMinRun) cuts.push_back(q);
-    }
-    cuts.push_back(b1);
-    for (size_t c = 0; c + 1 < cuts.size(); ++c) {
-      LevelLaunch lv;
-      lv.begin = cuts[c];
-      lv.count = cuts[c + 1] - cuts[c];
-      for (int32_t q = lv.begin; q < lv.begin + lv.count; ++q) {
-        const int32_t f = fp_.level_fronts[q];
-        lv.max_fsz = std::max(lv.max_fsz, fp_.fsz[f]);
-        lv.max_nc = std::max(lv.max_nc, fp_.nc[f]);
-        lv.max_src = std::max<int>(lv.max_src, (int)(fp_.fe_ptr[f + 1] - fp_.fe_ptr[f]));
-      }
-      d.levels.push_back(lv);
-    }
-  }
+  std::vector<std::vector<int32_t>> by_level(fp_.num_levels);
+  for (int32_t L = 0; L < fp_.num_levels; ++L)
+    by_level[L].assign(fp_.level_fronts.begin() + fp_.level_ptr[L], fp_.level_fronts.begin() + fp_.level_ptr[L + 1]);
+  d.levels = level_launches(by_level);
+  d.task_sets.clear();
+  d.ts = nullptr;
   assign_tiers(cfg_.tc_min_front > 0 ? cfg_.tc_min_front : kTcDefaultMinFront);
   // The top of the tree for the backward sweep: the trailing levels of at
   // most kBackwardTopFronts fronts.
@@ -456,28 +583,7 @@ void Engine::upload_plan() {
     }
   }
   // source lists in launch order, each padded to its launch's longest
-  {
-    std::vector<long long> psrc;
-    std::vector<int32_t> pdst;
-    for (auto& lv : d.levels) {
-      lv.max_src = std::max(lv.max_src, 1);
-      lv.fe_base = (long long)psrc.size();
-      for (int32_t q = lv.begin; q < lv.begin + lv.count; ++q) {
-        const int32_t f = fp_.level_fronts[q];
-        const int64_t a = fp_.fe_ptr[f], z = fp_.fe_ptr[f + 1];
-        for (int64_t e = a; e < z; ++e) {
-          psrc.push_back(fp_.fe_src[e]);
-          pdst.push_back(fp_.fe_dst[e]);
-        }
-        for (int64_t e = z - a; e < lv.max_src; ++e) {
-          psrc.push_back(0);
-          pdst.push_back(-1);
-        }
-      }
-    }
-    d.fe_src.upload(psrc);
-    d.fe_dst.upload(pdst);
-  }
+  pad_lists(d.levels, fp_.level_fronts, d.fe_src, d.fe_dst);
   // the front tree in level order for the single-system launch: each front's
   // parent and child count (the assembly's children are the tree's), and
   // where its list starts in the padded lists
@@ -567,6 +673,8 @@ void Engine::analyze_host(int32_t n_bus, const int32_t* indptr, const int32_t* i
   so.par_nd_base_large = cfg_.par_nd_base_large;
   sp_ = analyze_symbolic(ja_.dim, ja_.row_ptr.data(), ja_.col_idx.data(), so);
   fp_ = build_factor_program(sp_);
+  d_->task_sets.clear();
+  d_->ts = nullptr;
 }
 
 void Engine::analyze_matrix_host(int32_t n, int32_t nnz, const int32_t* row_ptr, const int32_t* col_idx) {
@@ -588,6 +696,8 @@ void Engine::analyze_matrix_host(int32_t n, int32_t nnz, const int32_t* row_ptr,
   so.par_nd_base_large = cfg_.par_nd_base_large;
   sp_ = analyze_symbolic(n, row_ptr, col_idx, so);
   fp_ = build_factor_program(sp_);
+  d_->task_sets.clear();
+  d_->ts = nullptr;
 }
 
 void Engine::initialize_matrix(int32_t n, int32_t nnz, const int32_t* row_ptr, const int32_t* col_idx) {
@@ -607,6 +717,8 @@ void Engine::initialize_matrix(int32_t n, int32_t nnz, const int32_t* row_ptr, c
   so.par_nd_base_large = cfg_.par_nd_base_large;
   sp_ = analyze_symbolic(n, row_ptr, col_idx, so);
   fp_ = build_factor_program(sp_);
+  d_->task_sets.clear();
+  d_->ts = nullptr;
   upload_plan();
   initialized_ = true;
   adjoint_ready_ = false;
@@ -619,6 +731,7 @@ void Engine::ensure_workspace(int32_t B) {
   const int Bp = (B + kWarp - 1) / kWarp * kWarp;
   d.B = B;
   d.Bp = Bp;
+  select_tasks();
   if (Bp > d.Bp_cap) {
     const size_t n = ja_.n_bus, dim = ja_.dim;
     const size_t es = factor_is_double() ? sizeof(double) : sizeof(float);
@@ -638,6 +751,9 @@ void Engine::ensure_workspace(int32_t B) {
     d.CB.reserve((size_t)std::max<int64_t>(fp_.cb_total, 1) * Bp * es);
     d.Y.reserve(dim * Bp * es);
     d.X.reserve(dim * Bp * es);
+    // the subtree tasks leave the padding scenarios alone; their state only
+    // has to stay finite
+    CUPF_CUDA(cudaMemset(d.X.p, 0, d.X.bytes));
     // dense fronts of levels too large for shared memory (and every wide-tier
     // front) live in global scratch; one launch at a time uses it
     size_t scratch = 0;
@@ -770,6 +886,7 @@ namespace {
 template <typename Set, typename Launch>
 bool choose_block_shapes(size_t n, const std::vector<int>& cand, Set set, Launch launch, cudaStream_t s,
                          const char* what) {
+  if (n == 0) return false;
   const size_t nc = cand.size();
   std::vector<double> t((nc + 1) * n, 1e30);  // [candidate 0..nc-1, rule = nc][launch]
   std::vector<cudaEvent_t> ev(n + 1, nullptr);
@@ -875,7 +992,7 @@ void Engine::autotune_factor(cudaStream_t s, const void* J) {
         double ms_t = 1e30;
         for (int rep = 0; rep < 3; ++rep) {
           CUPF_CUDA(cudaEventRecord(e0, s));
-          for (const auto& lv : d.levels) launch_factor_level<T, T>(lv, a, s);
+          launch_factor<T>(a, s);
           CUPF_CUDA(cudaEventRecord(e1, s));
           CUPF_CUDA(cudaEventSynchronize(e1));
           float ms = 0.f;
@@ -908,16 +1025,20 @@ void Engine::autotune_factor(cudaStream_t s, const void* J) {
   for (int p : {1, 2})
     for (int w : {1, 2, 4, 8}) cand.push_back(w + 256 * p);
   for (int w : {8, 16, 32}) cand.push_back(w + 256 * 3);
+  const bool tasks = use_tasks();
+  std::vector<LevelLaunch>& levels = tasks ? d.ts->rest : d.levels;
+  const FactorArgs<T, T> la = tasks ? rest_args<T>(a) : a;
+  if (tasks) launch_factor<T>(a, s);  // (the level launches read the tasks' contribution blocks)
   choose_block_shapes(
-      d.levels.size(), cand,
+      levels.size(), cand,
       [&](size_t i, int code) {
-        LevelLaunch& lv = d.levels[i];
+        LevelLaunch& lv = levels[i];
         int w = code & 0xff, p = code >> 8;
         if (p == 3 && !(lv.tier == 1 || wide_option(lv))) w = p = 0;
         lv.warps = w;
         lv.placement = lv.tier == 0 ? p : 0;
       },
-      [&](size_t i) { launch_factor_level<T, T>(d.levels[i], a, s); }, s, "factor");
+      [&](size_t i) { launch_factor_level<T, T>(levels[i], la, s); }, s, "factor");
   d.tuned_Bp = d.Bp;
   d.tuned_double = dbl;
   d.tuned_single = false;
@@ -965,6 +1086,31 @@ SweepArgs<T> Engine::sweep_args() const {
   return a;
 }
 
+std::vector<int32_t> Engine::task_array(std::string name) const {
+  int cls = 3;  // "name:class"
+  const size_t colon = name.find(':');
+  if (colon != std::string::npos) {
+    cls = std::min(std::max(std::atoi(name.c_str() + colon + 1), 0), 3);
+    name.resize(colon);
+  }
+  const TaskSet& set = task_set(cls);
+  const TaskPlan& t = set.tasks;
+  if (name == "task_meta") return t.meta;
+  if (name == "task_words") return t.words;
+  if (name == "task_sweep_meta") return set.sweeps.meta;
+  if (name == "task_sweep_words") return set.sweeps.words;
+  if (name == "task_sweep_stages") {
+    std::vector<int32_t> st;
+    for (const auto& s : set.sweeps.stages)
+      st.insert(st.end(), {s.begin, s.count, s.max_words, s.max_local, s.max_arena, s.max_rows, s.max_u, s.max_l,
+                           s.warps});
+    return st;
+  }
+  std::vector<int32_t> st;
+  for (const auto& s : t.stages) st.insert(st.end(), {s.begin, s.count, s.max_words, s.max_arena, s.warps});
+  return st;
+}
+
 std::vector<int32_t> Engine::factor_level_warps() const {
   std::vector<int32_t> w;
   for (const auto& lv : d_->levels) w.push_back(lv.warps);
@@ -1008,20 +1154,54 @@ void Engine::factor_all(cudaStream_t s, int store_l, const void* J) {
   auto& d = *d_;
   const FactorArgs<T, T> a = factor_args<T>(store_l, J);
   stage_begin(2, s);
-  if (single_tree(sizeof(T))) {
-    factor_tree<T>(a, s);
-    debug_check(s, "factor tree");
-    ++launches_;
-    ++d.stage_launches[2];
-  } else {
+  const int64_t n = launch_factor<T>(a, s);
+  launches_ += n;
+  d.stage_launches[2] += n;
+  stage_end(2, s);
+}
+
+// The whole factorization: the subtree tasks and the level launches of the
+// fronts they leave, or the single-system tree launch, or every level.
+// Returns the launches made.
+template <typename T>
+int64_t Engine::launch_factor(const FactorArgs<T, T>& a, cudaStream_t s) {
+  auto& d = *d_;
+  int64_t n = 0;
+  if (!use_tasks()) {
+    if (single_tree(sizeof(T))) {
+      factor_tree<T>(a, s);
+      debug_check(s, "factor tree");
+      return 1;
+    }
     for (const auto& lv : d.levels) {
       launch_factor_level<T, T>(lv, a, s);
       debug_check(s, "factor level");
-      ++launches_;
-      ++d.stage_launches[2];
+      ++n;
     }
+    return n;
   }
-  stage_end(2, s);
+  for (const auto& st : d.ts->tasks.stages) {
+    launch_factor_stage<T>(st, a, d.ts->task_meta.template as<int>(), d.ts->task_words.template as<int>(), d.task_lanes(), s);
+    debug_check(s, "factor tasks");
+    ++n;
+  }
+  const FactorArgs<T, T> r = rest_args<T>(a);
+  for (const auto& lv : d.ts->rest) {
+    launch_factor_level<T, T>(lv, r, s);
+    debug_check(s, "factor level");
+    ++n;
+  }
+  return n;
+}
+
+// The same arguments for the level launches of the fronts no task covers.
+template <typename T>
+FactorArgs<T, T> Engine::rest_args(FactorArgs<T, T> a) const {
+  const auto& d = *d_;
+  a.plan.front_meta = d.ts->rest_meta.as<int>();
+  a.plan.fe_src = d.ts->rest_src.as<long long>();
+  a.plan.fe_dst = d.ts->rest_dst.as<int>();
+  return a;
 }
 
 template <typename T>
@@ -1033,6 +1213,22 @@ void Engine::backward_all(cudaStream_t s) {
   launches_ += n;
   d.stage_launches[3] += n;
   stage_end(3, s);
+}
+
+bool Engine::use_sweep_tasks() const { return !d_->ts->sweeps.stages.empty(); }
+
+// One sweep over the subtree tasks (modes: launch_sweep_stage), a launch per stage.
+template <typename T>
+int64_t Engine::sweep_tasks(int mode, const SweepTaskArgs<T>& a, cudaStream_t s) {
+  auto& d = *d_;
+  const SweepPlan& sp = d.ts->sweeps;
+  const int n = (int)sp.stages.size();
+  for (int i = 0; i < n; ++i) {
+    launch_sweep_stage<T>(mode, sp.stages[mode < 2 ? i : n - 1 - i], a, d.Bp / kWarp, d.ts->sweep_meta.template as<int>(),
+                          d.ts->sweep_words.template as<int>(), d.task_lanes(), s);
+    debug_check(s, "sweep tasks");
+  }
+  return n;
 }
 
 // Backward substitution over the whole tree, root first: the narrow top in
@@ -1084,7 +1280,7 @@ void Engine::ensure_loop_graph(const DevState& st) {
   auto& d = *d_;
   const bool dbl = std::is_same<T, double>::value;
   if (d.exec && d.graph_Bp == d.Bp && d.graph_double == dbl && d.graph_yb == static_cast<const void*>(st.yb_re) &&
-      d.graph_single == single_system())
+      d.graph_single == single_system() && d.graph_lanes == d.task_lanes())
     return;
   if (d.exec) cudaGraphExecDestroy(d.exec);
   d.exec = nullptr;
@@ -1147,6 +1343,7 @@ void Engine::ensure_loop_graph(const DevState& st) {
   d.graph_Bp = d.Bp;
   d.graph_double = dbl;
   d.graph_single = single_system();
+  d.graph_lanes = d.task_lanes();
   d.graph_yb = st.yb_re;
   launches_ = before;
 }
@@ -1410,8 +1607,22 @@ void Engine::transpose_solve(const double* d_G, double* d_lam, cudaStream_t s) {
   a.TV = d.TV.as<T>();
   a.W = d.W.as<T>();
   a.Z = d.Z.as<T>();
-  for (const auto& lv : d.levels) launch_ut_forward_level<T>(lv, a, s);
-  for (int L = (int)d.levels.size() - 1; L >= 0; --L) launch_lt_backward_level<T>(d.levels[L], a, s);
+  if (use_sweep_tasks()) {
+    SweepTaskArgs<T> w;
+    w.Bp = d.Bp;
+    w.U = a.U;
+    w.L = a.L;
+    w.W = a.W;
+    w.X = a.Z;
+    w.TV = a.TV;
+    // J^T's right-hand side is indexed by Jacobian columns
+    launch_rows_to_permuted<T>(d.pl.col_perm, ja_.dim, d.Bp, d_G, a.W, s);
+    sweep_tasks<T>(1, w, s);
+    sweep_tasks<T>(2, w, s);
+  } else {
+    for (const auto& lv : d.levels) launch_ut_forward_level<T>(lv, a, s);
+    for (int L = (int)d.levels.size() - 1; L >= 0; --L) launch_lt_backward_level<T>(d.levels[L], a, s);
+  }
   // lambda is indexed by equation rows: undo the row ordering
   launch_permuted_to_rows<T>(d.pl.row_iperm, ja_.dim, d.Bp, d.Z.as<T>(), d_lam, s);
 }
@@ -1621,7 +1832,18 @@ void Engine::solve_values(const void* d_rhs, int32_t rhs_is_double, void* d_x, i
     a.G = d.G.as<double>();
     a.TV = d.TV.as<T>();
     a.W = d.W.as<T>();
-    for (const auto& lv : d.levels) launch_l_forward_level<T>(lv, a, s);
+    if (use_sweep_tasks()) {
+      SweepTaskArgs<T> w;
+      w.Bp = (int)Bp;
+      w.U = a.U;
+      w.L = a.L;
+      w.W = a.W;
+      w.TV = a.TV;
+      launch_rows_to_permuted<T>(d.pl.perm, (int)dim, (int)Bp, a.G, a.W, s);
+      sweep_tasks<T>(0, w, s);
+    } else {
+      for (const auto& lv : d.levels) launch_l_forward_level<T>(lv, a, s);
+    }
     SweepArgs<T> bk;
     bk.plan = d.pl;
     bk.groups = (int)Bp / kWarp;

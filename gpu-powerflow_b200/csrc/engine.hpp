@@ -123,6 +123,11 @@ class Engine {
   std::vector<int32_t> factor_level_tiers() const;
   // where each factor launch keeps its dense fronts: 1 shared memory, 2 the global scratch
   std::vector<int32_t> factor_level_placements() const;
+  // the factorization's subtree tasks (task_plan.hpp): "task_meta", "task_words",
+  // "task_stages" (per stage: first task, tasks, largest program and arena, warps of
+  // a team); the sweeps': "task_sweep_meta", "task_sweep_words",
+  // "task_sweep_stages"; ":c" after a name picks the batch class (default 3)
+  std::vector<int32_t> task_array(std::string name) const;
   int32_t tc_threshold() const { return tc_min_; }
   // the same for the backward sweep's launches, tree top first
   std::vector<int32_t> backward_launch_warps() const;
@@ -145,6 +150,7 @@ class Engine {
 
  private:
   struct Impl;
+  struct TaskSet;
   std::unique_ptr<Impl> d_;
   EngineConfig cfg_;
   JacobianAnalysis ja_;
@@ -165,6 +171,20 @@ class Engine {
 
   void ensure_workspace(int32_t B);
   void upload_plan();
+  TaskSet& task_set(int cls) const;
+  void select_tasks();
+  template <typename Buf>
+  void pad_lists(std::vector<LevelLaunch>& levels, const std::vector<int32_t>& order, Buf& src, Buf& dst) const;
+  std::vector<LevelLaunch> level_launches(const std::vector<std::vector<int32_t>>& by_level) const;
+  // the factorization runs as subtree tasks
+  bool use_tasks() const;
+  template <typename T>
+  int64_t launch_factor(const FactorArgs<T, T>& a, cudaStream_t s);
+  bool use_sweep_tasks() const;
+  template <typename T>
+  int64_t sweep_tasks(int mode, const SweepTaskArgs<T>& a, cudaStream_t s);
+  template <typename T>
+  FactorArgs<T, T> rest_args(FactorArgs<T, T> a) const;
   // factor kernel tier of every launch: the any-size tier from wide_min_front
   // rows, and with TF32 factors the tensor-core tier from tc_min rows
   void assign_tiers(int tc_min);

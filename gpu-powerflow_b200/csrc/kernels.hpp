@@ -239,6 +239,31 @@ inline size_t level_scratch_capacity(const LevelLaunch& lv, size_t elem_bytes, i
   return c;
 }
 
+// One stage of the subtree tasks (task_plan.hpp): its tasks' meta records and
+// programs on the device, lanes scenarios.
+struct TaskStage;
+template <typename T>
+void launch_factor_stage(const TaskStage& st, const FactorArgs<T, T>& a, const int* meta, const int* words, int lanes,
+                         cudaStream_t s);
+
+// Triangular sweeps over subtree tasks, one stage per launch: mode 0 L y = b
+// and 1 U^T w = g (stages leaves first, in place in W, update vectors between
+// tasks through TV), 2 L^T z = w (stages root first, W -> X).  Everything in
+// pivot order; groups: 32-scenario groups of the batch.
+struct SweepTaskStage;
+template <typename T>
+struct SweepTaskArgs {
+  int Bp = 0;
+  const T* U = nullptr;
+  const T* L = nullptr;
+  T* W = nullptr;
+  T* X = nullptr;
+  T* TV = nullptr;
+};
+template <typename T>
+void launch_sweep_stage(int mode, const SweepTaskStage& st, const SweepTaskArgs<T>& a, int groups,
+                        const int* meta, const int* words, int lanes, cudaStream_t s);
+
 template <typename T>
 struct SweepArgs {
   DevPlan plan;
@@ -247,6 +272,19 @@ struct SweepArgs {
   const T* Y = nullptr;
   T* X = nullptr;
 };
+
+// Warps per block of a level sweep launch: two where the level has many items
+// (fronts x scenario groups; at most 32 blocks are resident on an SM, so one
+// warp per block would leave half of its warp slots empty), up to 8 on the
+// narrow levels.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline int sweep_warps(long items) {
+  if (items >= 512) return 2;
+  if (items >= 128) return 4;
+  return 8;
+}
 
 template <typename T>
 struct AdjointSweepArgs {
@@ -309,6 +347,9 @@ void launch_copy_voltage_outputs(const DevGrid& g, const DevState& st, void* va_
 // adjoint helpers
 void launch_gather_adjoint_rhs(const DevGrid& g, const DevState& st, const void* grad_va, const void* grad_vm,
                                int is_double, double* G, cudaStream_t s);
+// W[k] = G[perm[k]]: a right-hand side into pivot order and the factor's type
+template <typename T>
+void launch_rows_to_permuted(const int* perm, int dim, int Bp, const double* G, T* W, cudaStream_t s);
 template <typename T>
 void launch_permuted_to_rows(const int* inv, int dim, int Bp, const T* Z, double* lam, cudaStream_t s);
 void launch_project_load_gradients(const DevGrid& g, const DevState& st, const double* lam, void* grad_p,

@@ -558,6 +558,16 @@ __global__ void k_permuted_to_rows(const int* __restrict__ inv, int dim, int Bp,
     lam[(size_t)f * Bp + b] = static_cast<double>(Z[(size_t)inv[f] * Bp + b]);
 }
 
+// W[k] = G[perm[k]]: a right-hand side in Jacobian order into pivot order
+template <typename T>
+__global__ void k_rows_to_permuted(const int* __restrict__ perm, int dim, int Bp, const double* __restrict__ G,
+                                   T* __restrict__ W) {
+  const int lane = threadIdx.x, wy = threadIdx.y;
+  const size_t b = (size_t)blockIdx.y * kWarp + lane;
+  for (int k = blockIdx.x * kRows + wy; k < dim; k += gridDim.x * kRows)
+    W[(size_t)k * Bp + b] = static_cast<T>(G[(size_t)perm[k] * Bp + b]);
+}
+
 // grad_load = -lambda at the bus's rows (adjoint_math.cpp:189-216)
 template <typename TO>
 __global__ void k_project_load_gradients(DevGrid g, DevState st, const double* __restrict__ lam, TO* grad_p,
@@ -883,6 +893,13 @@ void launch_gather_adjoint_rhs(const DevGrid& g, const DevState& st, const void*
   else
     k_gather_adjoint_rhs<float><<<rows_grid(g.dim, st.Bp), dim3(kWarp, kRows), 0, s>>>(g, st, grad_va, grad_vm, G);
 }
+
+template <typename T>
+void launch_rows_to_permuted(const int* perm, int dim, int Bp, const double* G, T* W, cudaStream_t s) {
+  k_rows_to_permuted<T><<<rows_grid(dim, Bp), dim3(kWarp, kRows), 0, s>>>(perm, dim, Bp, G, W);
+}
+template void launch_rows_to_permuted<float>(const int*, int, int, const double*, float*, cudaStream_t);
+template void launch_rows_to_permuted<double>(const int*, int, int, const double*, double*, cudaStream_t);
 
 template <typename T>
 void launch_permuted_to_rows(const int* inv, int dim, int Bp, const T* Z, double* lam, cudaStream_t s) {
