@@ -318,17 +318,36 @@ __global__ void k_transpose_bf16(const __nv_bfloat16* __restrict__ in, long long
   }
 }
 
+// The same for even sizes and 4-byte aligned rows, on 64 x 64 tiles: 128-byte
+// rows in and out instead of 64-byte ones.
+__global__ void k_transpose_bf16x2(const __nv_bfloat16* __restrict__ in, long long ld, __nv_bfloat16* __restrict__ out,
+                                   int rows, int cols) {
+  __shared__ __nv_bfloat162 t[64][33];
+  const int tx = threadIdx.x;
+  const int c = blockIdx.x * 64 + 2 * tx, r0 = blockIdx.y * 64;
+  for (int i = threadIdx.y; i < 64; i += 8)
+    if (r0 + i < rows && c < cols) t[i][tx] = *reinterpret_cast<const __nv_bfloat162*>(in + (size_t)(r0 + i) * ld + c);
+  __syncthreads();
+  const int r = r0 + 2 * tx;
+  for (int i = threadIdx.y; i < 64; i += 8) {
+    const int cc = blockIdx.x * 64 + i;
+    if (r >= rows || cc >= cols) continue;
+    const __nv_bfloat162 a = t[2 * tx][i / 2], b = t[2 * tx + 1][i / 2];
+    __nv_bfloat162 v;
+    v.x = i & 1 ? a.y : a.x;
+    v.y = i & 1 ? b.y : b.x;
+    *reinterpret_cast<__nv_bfloat162*>(out + (size_t)cc * rows + r) = v;
+  }
+}
+
 // features: x[b][k] = bf16((raw[b][k] - mean[k]) * inv_std[k]) for k < n_in, 0 for n_in <= k < width
 // (x has row stride ldx)
 __global__ void k_standardize(const float* __restrict__ raw, const float* __restrict__ mean,
                               const float* __restrict__ inv_std, __nv_bfloat16* __restrict__ x, long long ldx, int B,
                               int n_in, int width) {
-  const long long n = (long long)B * width;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const int k = (int)(i % width);
-    const long long b = i / width;
-    x[b * ldx + k] = __float2bfloat16(k < n_in ? (raw[b * n_in + k] - mean[k]) * inv_std[k] : 0.0f);
-  }
+  for (long long b = blockIdx.y; b < B; b += gridDim.y)
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < width; k += gridDim.x * blockDim.x)
+      x[b * ldx + k] = __float2bfloat16(k < n_in ? (raw[b * n_in + k] - mean[k]) * inv_std[k] : 0.0f);
 }
 
 // Power-flow load features, standardized, straight from Sbus: column k is
@@ -360,46 +379,106 @@ __global__ void k_load_features(const double* __restrict__ sbus, long long sbus_
 
 // mean-squared-error gradient on the first n_out columns:
 // g = 2 (pred - target) / (B n_out) in bf16 (0 in padding), loss += sum (pred - target)^2 / (B n_out)
-__global__ void k_mse_grad(const float* __restrict__ pred, int ld, const float* __restrict__ target, int n_out, int B,
-                           __nv_bfloat16* __restrict__ grad, float* __restrict__ loss) {
-  const long long n = (long long)B * ld;
+// A warp takes rows of the batch (no index division), and a block adds its
+// part of the loss with one atomic: one per warp and row would queue on the
+// single address.
+__global__ void __launch_bounds__(256)
+    k_mse_grad(const float* __restrict__ pred, int ld, const float* __restrict__ target, int n_out, int B,
+               __nv_bfloat16* __restrict__ grad, float* __restrict__ loss) {
+  __shared__ float part[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float scale = 1.0f / ((float)B * (float)n_out);
   float local = 0.0f;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const int k = (int)(i % ld);
-    const long long b = i / ld;
-    float gval = 0.0f;
-    if (k < n_out) {
-      const float d = pred[i] - target[b * n_out + k];
-      gval = 2.0f * d * scale;
-      local += d * d * scale;
+  // (row, 512-column chunk) pairs over the warps
+  const int chunks = (ld + 511) / 512;
+  for (long long i = (long long)blockIdx.x * 8 + warp; i < (long long)B * chunks; i += (long long)gridDim.x * 8) {
+    const long long b = i / chunks;
+    const int k0 = (int)(i - b * chunks) * 512, k1 = min(ld, k0 + 512);
+    const float* p = pred + b * ld;
+    const float* y = target + b * n_out;
+    __nv_bfloat16* g = grad + b * ld;
+#pragma unroll 8
+    for (int k = k0 + lane; k < k1; k += 32) {
+      float gval = 0.0f;
+      if (k < n_out) {
+        const float d = p[k] - y[k];
+        gval = 2.0f * d * scale;
+        local += d * d * scale;
+      }
+      g[k] = __float2bfloat16(gval);
     }
-    grad[i] = __float2bfloat16(gval);
   }
   for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
-  if ((threadIdx.x & 31) == 0 && loss) atomicAdd(loss, local);
+  if (lane == 0) part[warp] = local;
+  __syncthreads();
+  if (threadIdx.x == 0 && loss) {
+    for (int w = 1; w < 8; ++w) local += part[w];
+    atomicAdd(loss, local);
+  }
 }
 
 // column sums of a bf16 [rows][cols] matrix into fp32 [cols]
-__global__ void k_col_sum_bf16(const __nv_bfloat16* __restrict__ g, int rows, int cols, float* __restrict__ out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
+// (a block per 32 columns, its 32 warps share the rows; the partial sums are
+// added in warp order.  One thread per column walking all rows was a chain of
+// `rows` dependent loads on cols / 256 blocks.)
+__global__ void __launch_bounds__(1024)
+    k_col_sum_bf16(const __nv_bfloat16* __restrict__ g, int rows, int cols, float* __restrict__ out) {
+  __shared__ float part[32][33];
+  const int lane = threadIdx.x, warp = threadIdx.y;
+  const int c = blockIdx.x * 32 + lane;
   float s = 0.0f;
-  for (int r = 0; r < rows; ++r) s += __bfloat162float(g[(size_t)r * cols + c]);
-  out[c] = s;
+  if (c < cols) {
+#pragma unroll 8
+    for (int r = warp; r < rows; r += 32) s += __bfloat162float(g[(size_t)r * cols + c]);
+  }
+  part[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && c < cols) {
+    for (int w = 1; w < 32; ++w) s += part[w][lane];
+    out[c] = s;
+  }
 }
 
 // Adam on fp32 master weights; refreshes the bf16 copy used by the GEMMs.
+__device__ __forceinline__ void adam_step(float& w, float g, float& m, float& v, float lr, float b1, float b2,
+                                          float eps, float bc1, float bc2, float weight_decay) {
+  const float gi = g + weight_decay * w;
+  m = b1 * m + (1.0f - b1) * gi;
+  v = b2 * v + (1.0f - b2) * gi * gi;
+  w = w - lr * (m / bc1) / (sqrtf(v / bc2) + eps);
+}
+
+// Bound by memory (30 bytes a weight): four weights a thread where the arrays
+// are 16-byte aligned (w16: 8), so that a warp has 4 x 512 bytes in flight.
 __global__ void k_adam(float* __restrict__ w, const float* __restrict__ grad, float* __restrict__ m,
-                       float* __restrict__ v, __nv_bfloat16* __restrict__ w16, long long n, float lr, float b1,
+                       float* __restrict__ v, __nv_bfloat16* __restrict__ w16, long long n, int vec, float lr, float b1,
                        float b2, float eps, float bc1, float bc2, float weight_decay) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const float gi = grad[i] + weight_decay * w[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * gi;
-    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
+  const long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  const long long n4 = vec ? n / 4 : 0;
+  for (long long i = i0; i < n4; i += step) {
+    float4 wv = reinterpret_cast<float4*>(w)[i], mv = reinterpret_cast<float4*>(m)[i], vv = reinterpret_cast<float4*>(v)[i];
+    const float4 gv = reinterpret_cast<const float4*>(grad)[i];
+    adam_step(wv.x, gv.x, mv.x, vv.x, lr, b1, b2, eps, bc1, bc2, weight_decay);
+    adam_step(wv.y, gv.y, mv.y, vv.y, lr, b1, b2, eps, bc1, bc2, weight_decay);
+    adam_step(wv.z, gv.z, mv.z, vv.z, lr, b1, b2, eps, bc1, bc2, weight_decay);
+    adam_step(wv.w, gv.w, mv.w, vv.w, lr, b1, b2, eps, bc1, bc2, weight_decay);
+    reinterpret_cast<float4*>(m)[i] = mv;
+    reinterpret_cast<float4*>(v)[i] = vv;
+    reinterpret_cast<float4*>(w)[i] = wv;
+    if (w16) {
+      __nv_bfloat162 o[2];
+      o[0].x = __float2bfloat16(wv.x);
+      o[0].y = __float2bfloat16(wv.y);
+      o[1].x = __float2bfloat16(wv.z);
+      o[1].y = __float2bfloat16(wv.w);
+      reinterpret_cast<uint2*>(w16)[i] = *reinterpret_cast<const uint2*>(o);
+    }
+  }
+  for (long long i = 4 * n4 + i0; i < n; i += step) {
+    float wi = w[i], mi = m[i], vi = v[i];
+    adam_step(wi, grad[i], mi, vi, lr, b1, b2, eps, bc1, bc2, weight_decay);
     m[i] = mi;
     v[i] = vi;
-    const float wi = w[i] - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
     w[i] = wi;
     if (w16) w16[i] = __float2bfloat16(wi);
   }
@@ -613,6 +692,13 @@ int mlp_error_flag(int* out_host, int reset) {
 int mlp_transpose_bf16(const void* in, long long ld, void* out, int rows, int cols, void* stream) {
   return guarded([&] {
     if (ld < cols) throw std::invalid_argument("mlp_transpose_bf16: ld must be >= cols");
+    if (rows % 2 == 0 && cols % 2 == 0 && ld % 2 == 0 &&
+        ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 3) == 0) {
+      k_transpose_bf16x2<<<dim3((cols + 63) / 64, (rows + 63) / 64), dim3(32, 8), 0,
+                           static_cast<cudaStream_t>(stream)>>>(static_cast<const __nv_bfloat16*>(in), ld,
+                                                                static_cast<__nv_bfloat16*>(out), rows, cols);
+      return;
+    }
     dim3 grid((cols + 31) / 32, (rows + 31) / 32);
     k_transpose_bf16<<<grid, dim3(32, 8), 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const __nv_bfloat16*>(in), ld, static_cast<__nv_bfloat16*>(out), rows, cols);
@@ -623,7 +709,8 @@ int mlp_standardize(const float* raw, const float* mean, const float* inv_std, v
                     int n_in, int width, void* stream) {
   return guarded([&] {
     if (ldx < width || width < n_in) throw std::invalid_argument("mlp_standardize: need n_in <= width <= ldx");
-    k_standardize<<<grid1d((long long)B * width), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+    const dim3 grid((unsigned)std::max(1, std::min((width + 255) / 256, 4)), (unsigned)std::max(1, std::min(B, 16384)));
+    k_standardize<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
         raw, mean, inv_std, static_cast<__nv_bfloat16*>(x), ldx, B, n_in, width);
   });
 }
@@ -649,14 +736,14 @@ int mlp_load_features(const double* sbus, long long sbus_stride, const double* s
 int mlp_mse_grad(const float* pred, int ld, const float* target, int n_out, int B, void* grad, float* loss,
                  void* stream) {
   return guarded([&] {
-    k_mse_grad<<<grid1d((long long)B * ld), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+    k_mse_grad<<<kSMs * 8, 256, 0, static_cast<cudaStream_t>(stream)>>>(
         pred, ld, target, n_out, B, static_cast<__nv_bfloat16*>(grad), loss);
   });
 }
 
 int mlp_col_sum_bf16(const void* g, int rows, int cols, float* out, void* stream) {
   return guarded([&] {
-    k_col_sum_bf16<<<(cols + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+    k_col_sum_bf16<<<(cols + 31) / 32, dim3(32, 32), 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const __nv_bfloat16*>(g), rows, cols, out);
   });
 }
@@ -665,8 +752,11 @@ int mlp_adam(float* w, const float* grad, float* m, float* v, void* w_bf16, long
              float eps, int step, float weight_decay, void* stream) {
   return guarded([&] {
     const float bc1 = 1.0f - std::pow(b1, (float)step), bc2 = 1.0f - std::pow(b2, (float)step);
+    const uintptr_t all = reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(grad) |
+                          reinterpret_cast<uintptr_t>(m) | reinterpret_cast<uintptr_t>(v);
+    const int vec = (all & 15) == 0 && (reinterpret_cast<uintptr_t>(w_bf16) & 7) == 0;
     k_adam<<<grid1d(n), 256, 0, static_cast<cudaStream_t>(stream)>>>(w, grad, m, v, static_cast<__nv_bfloat16*>(w_bf16),
-                                                                      n, lr, b1, b2, eps, bc1, bc2, weight_decay);
+                                                                      n, vec, lr, b1, b2, eps, bc1, bc2, weight_decay);
   });
 }
 
