@@ -235,10 +235,13 @@ bool Engine::single_system() const { return cfg_.batch1_schedule == 0 && d_->B =
 
 bool Engine::use_tasks() const {
   if (d_->ts->tasks.stages.empty() || (d_->B == 1 && cfg_.batch1_schedule == 1)) return false;
-  // a single small system: one tree launch costs less than a launch per stage
-  // (118 buses, 94 fronts: 464 against 500 us per graph-mode solve; 2,000
-  // buses, 1,671 fronts: 1,265 against 1,125 us)
-  return !single_system() || (d_->ts->rest.empty() && fp_.P >= 256);
+  // Small trees are a few short levels, and the stages' launches cost as much
+  // as the levels': per graph-mode iteration 94 against 113 us by levels and
+  // by tasks with 100 buses (about 75 fronts) x 64, 127 against 126 us with
+  // 300 buses (about 250 fronts), 220 against 185 us with 1,000.  For a single
+  // system the other way is one launch over the whole tree.
+  if (single_system() && !d_->ts->rest.empty()) return false;
+  return fp_.P >= 300;
 }
 
 // The single-system factorization as one tree launch: batch 1, no
@@ -1302,7 +1305,7 @@ void Engine::ensure_loop_graph(const DevState& st) {
     CUPF_CUDA(cudaStreamBeginCaptureToGraph(cs, graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     capturing = true;
     launch_ibus_mismatch(d.g, st, cs);
-    launch_loop_check(h, ctl, norm, fin, cs);
+    launch_loop_check(h, ctl, norm, fin, st.Bp, cs);
     cudaStreamCaptureStatus cst;
     cudaGraph_t cap = nullptr;
     const cudaGraphNode_t* deps = nullptr;
@@ -1326,7 +1329,7 @@ void Engine::ensure_loop_graph(const DevState& st) {
     iteration_tail<T>(cs, 0);
     d.graph_body_launches = (launches_ - b0) + 2;
     launch_ibus_mismatch(d.g, st, cs);
-    launch_loop_check(h, ctl, norm, fin, cs);
+    launch_loop_check(h, ctl, norm, fin, st.Bp, cs);
     capturing = false;
     CUPF_CUDA(cudaStreamEndCapture(cs, &done));
     CUPF_CUDA(cudaGraphInstantiate(&d.exec, graph, 0));

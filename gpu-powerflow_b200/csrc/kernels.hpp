@@ -389,7 +389,7 @@ void launch_ctl_load(const LoopCtl* host_ctl, LoopCtl* ctl, cudaStream_t s);
 void launch_ctl_store(const LoopCtl* ctl, LoopCtl* host_ctl, const double* final_norm, double* host_final,
                       double* d_final, int B, cudaStream_t s);
 void launch_loop_check(cudaGraphConditionalHandle h, LoopCtl* ctl, const unsigned long long* norm_bits,
-                       double* final_norm, cudaStream_t s);
+                       double* final_norm, int Bp, cudaStream_t s);
 void launch_sumsq2(const double* R, const double* G, int dim, int B, int Bp, double* scratch, cudaStream_t s);
 // [B][rows] (TS) -> [rows][Bp] (TD) and back; pad scenarios copy scenario B - 1
 template <typename TS, typename TD>

@@ -6,6 +6,7 @@
 // indices are warp-uniform broadcasts and the state accesses are coalesced.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 
@@ -760,10 +761,15 @@ __global__ void k_ybus_to_rows(const double* __restrict__ yc, long long stride, 
   }
 }
 
+// Rows (entries) per warp: four where the grid fills the GPU (one per warp
+// took the 2,000-bus x 1,024 mismatch from 49 to 50 us and the fill from 62 to
+// 66), one where it does not: a warp's rows are dependent chains of loads one
+// after the other, and that chain is then the kernel's whole time.
 dim3 rows_grid(int rows, int Bp) {
-  int bx = (rows + kRows * 4 - 1) / (kRows * 4);
-  if (bx < 1) bx = 1;
-  return dim3(bx, Bp / kWarp);
+  const int groups = Bp / kWarp;
+  int per = kRows * 4;
+  if ((long)((rows + per - 1) / per) * groups < 2 * 148) per = kRows;
+  return dim3(std::max(1, (rows + per - 1) / per), groups);
 }
 
 }  // namespace
@@ -959,8 +965,10 @@ void launch_ybus_to_rows(const double* yc, long long stride, int nnz, int B, int
 }
 
 void launch_loop_check(cudaGraphConditionalHandle h, LoopCtl* ctl, const unsigned long long* norm_bits,
-                       double* final_norm, cudaStream_t s) {
-  k_loop_check<<<1, kCheckThreads, 0, s>>>(h, ctl, norm_bits, final_norm);
+                       double* final_norm, int Bp, cudaStream_t s) {
+  const int threads = std::min(kCheckThreads, Bp);
+  // (a small batch needs no more warps than its scenarios fill)
+  k_loop_check<<<1, threads, 0, s>>>(h, ctl, norm_bits, final_norm);
 }
 
 namespace {
