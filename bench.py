@@ -53,7 +53,7 @@ MAX_ITER = 10
 
 
 # DRAM traffic (read + write) of one Mixed factorization of the 2,000-bus
-# grid, per 1,024 scenarios: its 19 level launches captured with ncu at 256
+# grid, per 1,024 scenarios: a launch per level, captured with ncu at 256
 # scenarios (72.2 MB read; the writes stay in L2 at that size), scaled by 4
 # (the read traffic grows with the batch; a capture at 1,024 scenarios read
 # 278.8 MB and wrote 11.9 MB)
@@ -593,7 +593,7 @@ def run_engine(args) -> None:
                     "serial": {"value": round(e2e_serial_value, 1), "ms_per_step": round(ms_e2e_serial, 4),
                                "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                                "method": "upload, solve, download one after the other"}},
-            "roofline": {"kernel": "k_front_factor (all level launches of one factorization)", "bound": "hbm",
+            "roofline": {"kernel": "k_factor_tasks (all launches of one factorization)", "bound": "hbm",
                          "achieved": round(achieved, 1), "peak": peaks["hbm_gbs"], "unit": "GB/s",
                          "frac": round(achieved / peaks["hbm_gbs"], 4), "traffic": traffic,
                          "algorithmic_bytes": fbytes, "ms_per_factorization": round(per_fact_ms, 4),
@@ -777,7 +777,7 @@ def run_extras(args, dev) -> dict:
                 th.append((time.perf_counter() - t0) * 1e3)
             s1[name] = {"device_ms": round(statistics.median(ts), 4), "host_api_ms": round(statistics.median(th), 4),
                         "iterations": int(it1), "converged": bool(r1.converged_numpy.all())}
-        out[key] = {**s1, "method": "batch of 1 (single-system schedule: the factorization as one launch over "
+        out[key] = {**s1, "method": "batch of 1 (single-system schedule: a tree launch or subtree tasks over "
                                   "the front tree); median of 50 solves"}
     return out
 
