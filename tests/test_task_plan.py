@@ -293,10 +293,10 @@ def test_task_programs_of_a_reference_system(limit):
 @pytest.mark.gpu
 @pytest.mark.parametrize("precision,tol", [(cupf.CustomPrecision.FP64, 1e-12), (cupf.CustomPrecision.FP32, 2e-4)])
 @pytest.mark.parametrize("n", [1, 3, 24, 70, 130])
-def test_dense_systems_take_every_route(n, precision, tol):
-    """Dense diagonally dominant systems: fronts of up to 24 rows factor and
-    sweep as tasks, 70 rows factor on the level launches and sweep as tasks,
-    130 rows also sweep level by level.  Residuals to the rounding of an LU of
+def test_dense_systems_factor_and_solve(n, precision, tol):
+    """Dense diagonally dominant systems of one chain of fronts, up to 130 rows:
+    small trees, on the single-system tree, the level launches and, from 65
+    rows on, the any-size tier.  Residuals to the rounding of an LU of
     these matrices (condition below 10; n x the unit roundoff x a factor of
     about 50)."""
     import torch
