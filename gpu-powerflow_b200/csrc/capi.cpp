@@ -786,6 +786,16 @@ pf_status pf_plan_array64(pf_handle h, const char* name, int64_t* out, int64_t c
   if (n == "u_off") v = &fp.u_off;
   if (n == "l_off") v = &fp.l_off;
   if (n == "cb_off") v = &fp.cb_off;
+  std::vector<int64_t> norms;
+  if (n == "mismatch_norm_bits") {
+    try {
+      norms = h->eng->mismatch_norm_bits();
+    } catch (const std::exception& e) {
+      h->err = e.what();
+      return PF_RUNTIME_ERROR;
+    }
+    v = &norms;
+  }
   if (!v) {
     h->err = "unknown int64 plan array: " + n;
     return PF_INVALID_ARGUMENT;

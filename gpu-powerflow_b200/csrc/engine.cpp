@@ -118,6 +118,7 @@ struct Engine::Impl {
   std::map<int, std::unique_ptr<TaskSet>> task_sets;
   TaskSet* ts = nullptr;  // of the current batch
   int graph_lanes = 0;    // tasks' scenarios of the captured solve
+  int single_batch() const { return B == 1 ? 1 : 0; }
   int task_lanes() const { return B == 1 ? 1 : Bp; }  // scenarios the tasks cover (padding included)
   // backward sweep: the narrow top levels (launch-list entries from bw_first
   // on) run as one launch over bw_bounds (descending level boundaries)
@@ -754,9 +755,6 @@ void Engine::ensure_workspace(int32_t B) {
     d.CB.reserve((size_t)std::max<int64_t>(fp_.cb_total, 1) * Bp * es);
     d.Y.reserve(dim * Bp * es);
     d.X.reserve(dim * Bp * es);
-    // the subtree tasks leave the padding scenarios alone; their state only
-    // has to stay finite
-    CUPF_CUDA(cudaMemset(d.X.p, 0, d.X.bytes));
     // dense fronts of levels too large for shared memory (and every wide-tier
     // front) live in global scratch; one launch at a time uses it
     size_t scratch = 0;
@@ -1083,6 +1081,7 @@ SweepArgs<T> Engine::sweep_args() const {
   a.plan = d.pl;
   a.groups = d.Bp / kWarp;
   a.Bp = d.Bp;
+  a.single = d.single_batch();
   a.U = d.U.as<T>();
   a.Y = d.Y.as<T>();
   a.X = d.X.as<T>();
@@ -1608,6 +1607,7 @@ void Engine::transpose_solve(const double* d_G, double* d_lam, cudaStream_t s) {
   a.plan = d.pl;
   a.groups = d.Bp / kWarp;
   a.Bp = d.Bp;
+  a.single = d.single_batch();
   a.U = d.U.as<T>();
   a.L = d.L.as<T>();
   a.G = d_G;
@@ -1631,7 +1631,7 @@ void Engine::transpose_solve(const double* d_G, double* d_lam, cudaStream_t s) {
     for (int L = (int)d.levels.size() - 1; L >= 0; --L) launch_lt_backward_level<T>(d.levels[L], a, s);
   }
   // lambda is indexed by equation rows: undo the row ordering
-  launch_permuted_to_rows<T>(d.pl.row_iperm, ja_.dim, d.Bp, d.Z.as<T>(), d_lam, s);
+  launch_permuted_to_rows<T>(d.pl.row_iperm, ja_.dim, d.Bp, d.single_batch(), d.Z.as<T>(), d_lam, s);
 }
 
 double Engine::solve_adjoint_device(const void* grad_va, const void* grad_vm, void* grad_p, void* grad_q,
@@ -1834,6 +1834,7 @@ void Engine::solve_values(const void* d_rhs, int32_t rhs_is_double, void* d_x, i
     a.plan = d.pl;
     a.groups = (int)Bp / kWarp;
     a.Bp = (int)Bp;
+    a.single = d.single_batch();
     a.U = d.U.as<T>();
     a.L = d.L.as<T>();
     a.G = d.G.as<double>();
@@ -1855,12 +1856,13 @@ void Engine::solve_values(const void* d_rhs, int32_t rhs_is_double, void* d_x, i
     bk.plan = d.pl;
     bk.groups = (int)Bp / kWarp;
     bk.Bp = (int)Bp;
+    bk.single = d.single_batch();
     bk.U = d.U.as<T>();
     bk.Y = d.W.as<T>();
     bk.X = d.X.as<T>();
     backward_levels<T>(bk, s);
     // x is indexed by columns: undo the column ordering
-    launch_permuted_to_rows<T>(d.pl.iperm, (int)dim, (int)Bp, d.X.as<T>(), d.lam.as<double>(), s);
+    launch_permuted_to_rows<T>(d.pl.iperm, (int)dim, (int)Bp, d.single_batch(), d.X.as<T>(), d.lam.as<double>(), s);
   };
   if (dbl) run(double{});
   else run(float{});
@@ -1901,6 +1903,14 @@ void Engine::evaluate_host(const double* V, const double* sbus, int32_t B, doubl
   CUPF_CUDA(cudaMemcpyAsync(J_out, d.G.p, (size_t)ja_.nnz * B * 8, cudaMemcpyDeviceToHost, s));
   CUPF_CUDA(cudaStreamSynchronize(s));
   CUPF_CUDA(cudaGetLastError());
+}
+
+std::vector<int64_t> Engine::mismatch_norm_bits() const {
+  std::vector<int64_t> out(d_->norm.p ? d_->Bp : 0);
+  if (out.empty()) return out;
+  CUPF_CUDA(cudaStreamSynchronize(d_->own));
+  CUPF_CUDA(cudaMemcpy(out.data(), d_->norm.p, out.size() * sizeof(int64_t), cudaMemcpyDeviceToHost));
+  return out;
 }
 
 std::vector<int32_t> Engine::singular_flags() const {

@@ -138,6 +138,9 @@ class Engine {
   bool factor_is_double() const;
   bool adjoint_cache_valid() const { return adjoint_ready_; }
   int32_t cached_batch() const { return B_; }
+  // the norms of the last mismatch evaluation as the bits of doubles, one per
+  // column of the padded batch (the padding repeats the last scenario)
+  std::vector<int64_t> mismatch_norm_bits() const;
   std::vector<int32_t> singular_flags() const;  // per scenario of the last factorization
   // kernel launches issued by the last solve (for reporting)
   int64_t last_launches() const { return launches_; }

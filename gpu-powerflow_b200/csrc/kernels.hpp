@@ -268,6 +268,7 @@ template <typename T>
 struct SweepArgs {
   DevPlan plan;
   int groups = 0, Bp = 0;
+  int single = 0;  // a batch of one: U and Y are read in column 0 for all 32 columns of X
   const T* U = nullptr;
   const T* Y = nullptr;
   T* X = nullptr;
@@ -290,6 +291,7 @@ template <typename T>
 struct AdjointSweepArgs {
   DevPlan plan;
   int groups = 0, Bp = 0;
+  int single = 0;  // a batch of one: U and L are read in column 0
   const T* U = nullptr;
   const T* L = nullptr;
   const double* G = nullptr;  // rhs in Jacobian-row order
@@ -347,11 +349,12 @@ void launch_copy_voltage_outputs(const DevGrid& g, const DevState& st, void* va_
 // adjoint helpers
 void launch_gather_adjoint_rhs(const DevGrid& g, const DevState& st, const void* grad_va, const void* grad_vm,
                                int is_double, double* G, cudaStream_t s);
-// W[k] = G[perm[k]]: a right-hand side into pivot order and the factor's type
+// W[k] = G[perm[k]]: a right-hand side into pivot order and the factor's type;
+// back: lam[f] = Z[inv[f]] (single: a batch of one, column 0 of Z into every column)
 template <typename T>
 void launch_rows_to_permuted(const int* perm, int dim, int Bp, const double* G, T* W, cudaStream_t s);
 template <typename T>
-void launch_permuted_to_rows(const int* inv, int dim, int Bp, const T* Z, double* lam, cudaStream_t s);
+void launch_permuted_to_rows(const int* inv, int dim, int Bp, int single, const T* Z, double* lam, cudaStream_t s);
 void launch_project_load_gradients(const DevGrid& g, const DevState& st, const double* lam, void* grad_p,
                                    void* grad_q, int is_double, cudaStream_t s);
 // r = g - J^T lambda, J given by its CSR values [nnz_j][Bp] (fp64)

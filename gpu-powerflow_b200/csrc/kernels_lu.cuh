@@ -1002,18 +1002,24 @@ __global__ void __launch_bounds__(256)
 // One warp = one front x 32 scenarios.  The warp stages its front's U rows
 // (contiguous elements) and the x rows of its CB rows (gathered through
 // front_rows) with cp.async, then solves the nc pivots from shared memory.
+//
+// SINGLE: a batch of one.  Its subtree tasks (kernels_task.cuh) write column 0
+// of the factors and of y alone, so every lane reads that column, and the 31
+// padding columns of X get the scenario's own solution: the padding state
+// stays a copy of the scenario.  (A template: as a run-time flag it cost the
+// 2,000-bus x 1,024 solve 2 %, 2,746 -> 2,804 us.)
 // ---------------------------------------------------------------------------
 // One front x 32 scenarios (starting at col0), by one warp, with its
 // staging area Us.
 // STAGED = false (fronts whose U rows do not fit in shared memory): the same
 // substitution reading U and x straight from global memory.
-template <typename T, bool STAGED = true>
+template <typename T, bool STAGED, bool SINGLE>
 __device__ __forceinline__ void backward_front(const DevPlan& pl, const FrontMeta& m, size_t col0, int Bp, T* Us,
                                                const T* __restrict__ U, const T* __restrict__ Y,
                                                T* __restrict__ X) {
   constexpr int kPieces = kWarp * sizeof(T) / 16;
-  const int lane = threadIdx.x & 31;
-  const size_t b = col0 + lane;
+  const int lane = threadIdx.x & 31, ulane = SINGLE ? 0 : lane;
+  const size_t b = col0 + lane, ub = col0 + ulane;
   const int fs = m.fs, nc = m.nc, uc = fs - nc;
   const int fr0 = m.fr0, first = m.first;
   const long long uo = m.uo;
@@ -1021,17 +1027,18 @@ __device__ __forceinline__ void backward_front(const DevPlan& pl, const FrontMet
     // x_k = (y_k - sum_{j > k} u_kj x(row j)) / u_kk, k from the last pivot
     // down; the pivots' x rows are first + k, written by this thread
     for (int k = nc - 1; k >= 0; --k) {
-      const T* urow = U + (size_t)(uo + (long long)k * fs) * Bp + b;
-      T s = Y[(size_t)(first + k) * Bp + b];
+      const T* urow = U + (size_t)(uo + (long long)k * fs) * Bp + ub;
+      T s = Y[(size_t)(first + k) * Bp + ub];
       for (int j = k + 1; j < fs; ++j) s -= urow[(size_t)j * Bp] * X[(size_t)pl.front_rows[fr0 + j] * Bp + b];
       X[(size_t)(first + k) * Bp + b] = s / urow[(size_t)k * Bp];
     }
     return;
   }
   T* Xs = Us + (size_t)nc * fs * kWarp;  // [fs][32]
-  // U rows: contiguous elements uo .. uo + nc * fs
-  for (int t = lane; t < nc * fs * kPieces; t += kWarp) {
-    const int e = t / kPieces, piece = t % kPieces;
+  // U rows: contiguous elements uo .. uo + nc * fs (SINGLE: only the 16 bytes with column 0)
+  constexpr int kUPieces = SINGLE ? 1 : kPieces;
+  for (int t = lane; t < nc * fs * kUPieces; t += kWarp) {
+    const int e = t / kUPieces, piece = t % kUPieces;
     cp_async16(reinterpret_cast<unsigned char*>(Us + (size_t)e * kWarp) + piece * 16,
                reinterpret_cast<const unsigned char*>(U + (size_t)(uo + e) * Bp + col0) + piece * 16);
   }
@@ -1046,13 +1053,13 @@ __device__ __forceinline__ void backward_front(const DevPlan& pl, const FrontMet
   cp_async_commit();
   T yk[8];
 #pragma unroll
-  for (int k = 0; k < 8; ++k) yk[k] = k < nc ? Y[(size_t)(first + k) * Bp + b] : T(0);
+  for (int k = 0; k < 8; ++k) yk[k] = k < nc ? Y[(size_t)(first + k) * Bp + ub] : T(0);
   cp_async_wait<0>();
   __syncwarp();
 #pragma unroll
   for (int k = 7; k >= 0; --k) {
     if (k < nc) {
-      const T* urow = Us + (size_t)k * fs * kWarp + lane;
+      const T* urow = Us + (size_t)k * fs * kWarp + ulane;
       T s = yk[k];
       for (int j = k + 1; j < fs; ++j) s -= urow[(size_t)j * kWarp] * Xs[(size_t)j * kWarp + lane];
       const T xk = s / urow[(size_t)k * kWarp];
@@ -1063,7 +1070,7 @@ __device__ __forceinline__ void backward_front(const DevPlan& pl, const FrontMet
   __syncwarp();  // the staging area is reused by the warp's next front
 }
 
-template <typename T, bool STAGED = true>
+template <typename T, bool STAGED, bool SINGLE>
 __global__ void __launch_bounds__(256)
     k_backward_level(DevPlan pl, int level_begin, int level_count, int groups, int Bp, int warp_elems,
                      const T* __restrict__ U, const T* __restrict__ Y, T* __restrict__ X) {
@@ -1077,7 +1084,7 @@ __global__ void __launch_bounds__(256)
   const FrontMeta m = load_front_meta(pl.front_meta, q);  // (plan data: before the wait)
   chain_wait_previous();  // U, Y and the x of ancestors come from earlier kernels
   T* Us = reinterpret_cast<T*>(smem_raw) + (size_t)warp * warp_elems * kWarp;  // [nc * fs][32]
-  backward_front<T, STAGED>(pl, m, col0, Bp, Us, U, Y, X);
+  backward_front<T, STAGED, SINGLE>(pl, m, col0, Bp, Us, U, Y, X);
 }
 
 // The narrow top of the tree in one launch: block = one group of 32
@@ -1086,7 +1093,7 @@ __global__ void __launch_bounds__(256)
 // (the x a front reads come from its ancestors, written by this block).
 // lv_lo[t] .. lv_lo[t + 1]: level-order fronts of the t-th level from the
 // root (descending boundaries, nlev + 1 entries).
-template <typename T, bool STAGED = true>
+template <typename T, bool STAGED, bool SINGLE>
 __global__ void __launch_bounds__(256)
     k_backward_top(DevPlan pl, const int* __restrict__ lv_bounds, int nlev, int Bp, int warp_elems,
                    const T* __restrict__ U, const T* __restrict__ Y, T* __restrict__ X) {
@@ -1099,7 +1106,7 @@ __global__ void __launch_bounds__(256)
   for (int t = 0; t < nlev; ++t) {
     const int hi = lv_bounds[t], lo = lv_bounds[t + 1];
     for (int q = lo + warp; q < hi; q += W)
-      backward_front<T, STAGED>(pl, load_front_meta(pl.front_meta, q), col0, Bp, Us, U, Y, X);
+      backward_front<T, STAGED, SINGLE>(pl, load_front_meta(pl.front_meta, q), col0, Bp, Us, U, Y, X);
     __syncthreads();
   }
 }
@@ -1118,6 +1125,9 @@ __global__ void __launch_bounds__(256)
 // request, the values of 8 entries are requested together, and each row's
 // entries are summed in list order into ts[row * 32] (ts: this lane's column
 // of the block's [fs][32] area in shared memory; rows without entries get 0).
+//
+// single: a batch of one; every lane reads column 0 of the factors, the only
+// one its tasks write (backward_front).
 // ---------------------------------------------------------------------------
 template <typename T>
 __device__ __forceinline__ void gather_child_updates(const DevPlan& pl, int fr0, int r0, int r1, size_t b, int Bp,
@@ -1183,7 +1193,7 @@ __device__ __forceinline__ SweepItem sweep_item(const DevPlan& pl, int level_beg
 // Shared memory: [fs_cap][32] gathered rows, [8][32] pivot values.
 template <typename T, int NCMAX>
 __global__ void __launch_bounds__(256)
-    k_l_forward_level(DevPlan pl, int level_begin, int groups, int Bp, int fs_cap, const T* __restrict__ U,
+    k_l_forward_level(DevPlan pl, int level_begin, int groups, int Bp, int single, int fs_cap, const T* __restrict__ U,
                       const T* __restrict__ L, const double* __restrict__ G, T* __restrict__ TV,
                       T* __restrict__ Yo) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1191,7 +1201,7 @@ __global__ void __launch_bounds__(256)
   const int W = blockDim.x >> 5, warp = threadIdx.x >> 5;
   const SweepItem it = sweep_item(pl, level_begin, groups);
   const int fs = it.fs, nc = it.nc;
-  const size_t b = it.b;
+  const size_t b = it.b, fb = single ? 0 : b;
   const long long uo = pl.u_off[it.p], lo = pl.l_off[it.p], to = pl.tv_off[it.p];
   T* ts = reinterpret_cast<T*>(smem_raw) + (threadIdx.x & 31);
   T* ys = ts + (size_t)fs_cap * kWarp;
@@ -1206,7 +1216,7 @@ __global__ void __launch_bounds__(256)
       if (k < nc) {
         T s = static_cast<T>(G[(size_t)pl.perm[it.first + k] * Bp + b]) - ts[k * kWarp];
 #pragma unroll
-        for (int m = 0; m < k; ++m) s -= U[(size_t)(uo + (long long)k * fs + m) * Bp + b] * y[m];
+        for (int m = 0; m < k; ++m) s -= U[(size_t)(uo + (long long)k * fs + m) * Bp + fb] * y[m];
         y[k] = s;
         ys[k * kWarp] = s;
         Yo[(size_t)(it.first + k) * Bp + b] = s;
@@ -1222,7 +1232,7 @@ __global__ void __launch_bounds__(256)
     T s = ts[j * kWarp];
 #pragma unroll
     for (int m = 0; m < NCMAX; ++m)
-      if (m < nc) s += L[(size_t)(lo + (long long)(j - nc) * nc + m) * Bp + b] * y[m];
+      if (m < nc) s += L[(size_t)(lo + (long long)(j - nc) * nc + m) * Bp + fb] * y[m];
     TV[(size_t)(to + (j - nc)) * Bp + b] = s;
   }
 }
@@ -1236,14 +1246,14 @@ __global__ void __launch_bounds__(256)
 // ---------------------------------------------------------------------------
 template <typename T, int NCMAX>
 __global__ void __launch_bounds__(256)
-    k_ut_forward_level(DevPlan pl, int level_begin, int groups, int Bp, int fs_cap, const T* __restrict__ U,
+    k_ut_forward_level(DevPlan pl, int level_begin, int groups, int Bp, int single, int fs_cap, const T* __restrict__ U,
                        const double* __restrict__ G, T* __restrict__ TV, T* __restrict__ Wv) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   chain_allow_next();
   const int W = blockDim.x >> 5, warp = threadIdx.x >> 5;
   const SweepItem it = sweep_item(pl, level_begin, groups);
   const int fs = it.fs, nc = it.nc;
-  const size_t b = it.b;
+  const size_t b = it.b, fb = single ? 0 : b;
   const long long uo = pl.u_off[it.p], to = pl.tv_off[it.p];
   T* ts = reinterpret_cast<T*>(smem_raw) + (threadIdx.x & 31);
   T* wsm = ts + (size_t)fs_cap * kWarp;
@@ -1259,8 +1269,8 @@ __global__ void __launch_bounds__(256)
         // J^T's right-hand side is indexed by Jacobian columns
         T s = static_cast<T>(G[(size_t)pl.col_perm[it.first + k] * Bp + b]) - ts[k * kWarp];
 #pragma unroll
-        for (int m = 0; m < k; ++m) s -= U[(size_t)(uo + (long long)m * fs + k) * Bp + b] * w[m];
-        w[k] = s / U[(size_t)(uo + (long long)k * fs + k) * Bp + b];
+        for (int m = 0; m < k; ++m) s -= U[(size_t)(uo + (long long)m * fs + k) * Bp + fb] * w[m];
+        w[k] = s / U[(size_t)(uo + (long long)k * fs + k) * Bp + fb];
         wsm[k * kWarp] = w[k];
         Wv[(size_t)(it.first + k) * Bp + b] = w[k];
       }
@@ -1275,7 +1285,7 @@ __global__ void __launch_bounds__(256)
     T s = ts[j * kWarp];
 #pragma unroll
     for (int m = 0; m < NCMAX; ++m)
-      if (m < nc) s += U[(size_t)(uo + (long long)m * fs + j) * Bp + b] * w[m];
+      if (m < nc) s += U[(size_t)(uo + (long long)m * fs + j) * Bp + fb] * w[m];
     TV[(size_t)(to + (j - nc)) * Bp + b] = s;
   }
 }
@@ -1286,14 +1296,14 @@ __global__ void __launch_bounds__(256)
 // block with those partial sums (shared memory [W][8][32]).
 template <typename T, int NCMAX>
 __global__ void __launch_bounds__(256)
-    k_lt_backward_level(DevPlan pl, int level_begin, int groups, int Bp, const T* __restrict__ U,
+    k_lt_backward_level(DevPlan pl, int level_begin, int groups, int Bp, int single, const T* __restrict__ U,
                         const T* __restrict__ L, const T* __restrict__ Wv, T* __restrict__ Z) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   chain_allow_next();
   const int W = blockDim.x >> 5, warp = threadIdx.x >> 5;
   const SweepItem it = sweep_item(pl, level_begin, groups);
   const int fs = it.fs, nc = it.nc;
-  const size_t b = it.b;
+  const size_t b = it.b, fb = single ? 0 : b;
   const long long uo = pl.u_off[it.p], lo = pl.l_off[it.p];
   T* ps = reinterpret_cast<T*>(smem_raw) + (threadIdx.x & 31);
   chain_wait_previous();
@@ -1305,7 +1315,7 @@ __global__ void __launch_bounds__(256)
     const T zj = Z[(size_t)pl.front_rows[it.fr0 + j] * Bp + b];
 #pragma unroll
     for (int k = 0; k < NCMAX; ++k)
-      if (k < nc) acc[k] += L[(size_t)(lo + (long long)(j - nc) * nc + k) * Bp + b] * zj;
+      if (k < nc) acc[k] += L[(size_t)(lo + (long long)(j - nc) * nc + k) * Bp + fb] * zj;
   }
 #pragma unroll
   for (int k = 0; k < NCMAX; ++k) ps[(warp * NCMAX + k) * kWarp] = acc[k];
@@ -1319,7 +1329,7 @@ __global__ void __launch_bounds__(256)
         T s = Wv[(size_t)(it.first + k) * Bp + b];
 #pragma unroll
         for (int m = k + 1; m < NCMAX; ++m)
-          if (m < nc) s -= U[(size_t)(uo + (long long)m * fs + k) * Bp + b] * z[m];
+          if (m < nc) s -= U[(size_t)(uo + (long long)m * fs + k) * Bp + fb] * z[m];
         for (int w = 0; w < W; ++w) s -= ps[(w * NCMAX + k) * kWarp];
         z[k] = s;
         Z[(size_t)(it.first + k) * Bp + b] = s;
@@ -1378,8 +1388,10 @@ void launch_factor_t(const LevelLaunch& lv, const FactorArgs<T, TJ>& a, cudaStre
 // memory up front (outside any stream capture).
 template <typename T, typename TJ>
 void configure_front_kernels() {
-  allow_full_smem(reinterpret_cast<const void*>(k_backward_level<T>));
-  allow_full_smem(reinterpret_cast<const void*>(k_backward_top<T>));
+  allow_full_smem(reinterpret_cast<const void*>(k_backward_level<T, true, false>));
+  allow_full_smem(reinterpret_cast<const void*>(k_backward_level<T, true, true>));
+  allow_full_smem(reinterpret_cast<const void*>(k_backward_top<T, true, false>));
+  allow_full_smem(reinterpret_cast<const void*>(k_backward_top<T, true, true>));
 #define CUPF_ALLOW(F)                                                                  \
   allow_full_smem(reinterpret_cast<const void*>(k_front_factor<T, TJ, F, true>));    \
   allow_full_smem(reinterpret_cast<const void*>(k_front_factor<T, TJ, F, false>));
@@ -1516,7 +1528,7 @@ void launch_backward_level(const LevelLaunch& lv, const SweepArgs<T>& a, cudaStr
   const long items = (long)lv.count * a.groups;
   if (per_warp > kSmemLimit) {  // U rows too large to stage: read them from global memory
     const int w = lv.bw_wpb > 0 ? lv.bw_wpb : 4;
-    launch_chained(k_backward_level<T, false>, dim3((unsigned)((items + w - 1) / w)), dim3(w * kWarp), 0, s,
+    launch_chained(a.single ? k_backward_level<T, false, true> : k_backward_level<T, false, false>, dim3((unsigned)((items + w - 1) / w)), dim3(w * kWarp), 0, s,
                    "backward sweep", a.plan, lv.begin, lv.count, a.groups, a.Bp, warp_elems, a.U, a.Y, a.X);
     return;
   }
@@ -1526,7 +1538,7 @@ void launch_backward_level(const LevelLaunch& lv, const SweepArgs<T>& a, cudaStr
   wpb = std::max(1, std::min(wpb, 4));
   if (lv.bw_wpb > 0) wpb = std::min(lv.bw_wpb, cap);  // chosen by the engine's autotuner
   const size_t smem = per_warp * wpb;
-  auto kern = k_backward_level<T>;
+  auto kern = a.single ? k_backward_level<T, true, true> : k_backward_level<T, true, false>;
   allow_full_smem(reinterpret_cast<const void*>(kern));
   const unsigned blocks = (unsigned)((items + wpb - 1) / wpb);
   launch_chained(kern, dim3(blocks), dim3(wpb * kWarp), smem, s, "backward sweep", a.plan, lv.begin, lv.count,
@@ -1543,13 +1555,13 @@ void launch_backward_top(const LevelLaunch& top, const int* lv_bounds, int nlev,
   const size_t per_warp = (size_t)warp_elems * kWarp * sizeof(T);
   if (per_warp > kSmemLimit) {  // U rows too large to stage: read them from global memory
     const int w = top.bw_wpb > 0 ? top.bw_wpb : 4;
-    launch_chained(k_backward_top<T, false>, dim3((unsigned)a.groups), dim3(w * kWarp), 0, s,
+    launch_chained(a.single ? k_backward_top<T, false, true> : k_backward_top<T, false, false>, dim3((unsigned)a.groups), dim3(w * kWarp), 0, s,
                    "backward sweep (tree top)", a.plan, lv_bounds, nlev, a.Bp, warp_elems, a.U, a.Y, a.X);
     return;
   }
   const int cap = (int)std::min<size_t>(8, kSmemLimit / per_warp);
   const int wpb = top.bw_wpb > 0 ? std::min(top.bw_wpb, cap) : std::min(4, cap);
-  auto kern = k_backward_top<T>;
+  auto kern = a.single ? k_backward_top<T, true, true> : k_backward_top<T, true, false>;
   allow_full_smem(reinterpret_cast<const void*>(kern));
   launch_chained(kern, dim3((unsigned)a.groups), dim3(wpb * kWarp), per_warp * wpb, s, "backward sweep (tree top)",
                  a.plan, lv_bounds, nlev, a.Bp, warp_elems, a.U, a.Y, a.X);
@@ -1561,7 +1573,7 @@ void launch_ut_forward_level(const LevelLaunch& lv, const AdjointSweepArgs<T>& a
   if (lv.max_nc > 8) throw std::runtime_error("panels wider than 8 columns are not supported (max_panel_width <= 8)");
   const long items = (long)lv.count * a.groups;
   launch_sweep(k_ut_forward_level<T, 8>, items, sweep_warps(items), (size_t)(lv.max_fsz + 8) * kWarp * sizeof(T), s,
-               "adjoint sweep (U^T)", a.plan, lv.begin, a.groups, a.Bp, lv.max_fsz, a.U, a.G, a.TV, a.W);
+               "adjoint sweep (U^T)", a.plan, lv.begin, a.groups, a.Bp, a.single, lv.max_fsz, a.U, a.G, a.TV, a.W);
 }
 
 template <typename T>
@@ -1570,7 +1582,7 @@ void launch_l_forward_level(const LevelLaunch& lv, const AdjointSweepArgs<T>& a,
   if (lv.max_nc > 8) throw std::runtime_error("panels wider than 8 columns are not supported (max_panel_width <= 8)");
   const long items = (long)lv.count * a.groups;
   launch_sweep(k_l_forward_level<T, 8>, items, sweep_warps(items), (size_t)(lv.max_fsz + 8) * kWarp * sizeof(T), s,
-               "forward substitution", a.plan, lv.begin, a.groups, a.Bp, lv.max_fsz, a.U, a.L, a.G, a.TV, a.W);
+               "forward substitution", a.plan, lv.begin, a.groups, a.Bp, a.single, lv.max_fsz, a.U, a.L, a.G, a.TV, a.W);
 }
 
 template <typename T>
@@ -1580,7 +1592,7 @@ void launch_lt_backward_level(const LevelLaunch& lv, const AdjointSweepArgs<T>& 
   const long items = (long)lv.count * a.groups;
   const int warps = sweep_warps(items);
   launch_sweep(k_lt_backward_level<T, 8>, items, warps, (size_t)warps * 8 * kWarp * sizeof(T), s,
-               "adjoint sweep (L^T)", a.plan, lv.begin, a.groups, a.Bp, a.U, a.L, a.W, a.Z);
+               "adjoint sweep (L^T)", a.plan, lv.begin, a.groups, a.Bp, a.single, a.U, a.L, a.W, a.Z);
 }
 
 }  // namespace cupf_b200

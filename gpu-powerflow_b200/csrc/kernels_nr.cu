@@ -550,13 +550,15 @@ __global__ void k_gather_adjoint_rhs(DevGrid g, DevState st, const void* grad_va
 
 // lam[f] = Z[inv[f]]: a solution in pivot order back to Jacobian order
 // (inv = the column inverse for J x = b, the row inverse for J^T x = b)
+// single: a batch of one, whose sweep tasks write column 0 of Z alone; lam's
+// padding columns get copies of it.
 template <typename T>
-__global__ void k_permuted_to_rows(const int* __restrict__ inv, int dim, int Bp, const T* __restrict__ Z,
+__global__ void k_permuted_to_rows(const int* __restrict__ inv, int dim, int Bp, int single, const T* __restrict__ Z,
                                    double* __restrict__ lam) {
   const int lane = threadIdx.x, wy = threadIdx.y;
   const size_t b = (size_t)blockIdx.y * kWarp + lane;
   for (int f = blockIdx.x * kRows + wy; f < dim; f += gridDim.x * kRows)
-    lam[(size_t)f * Bp + b] = static_cast<double>(Z[(size_t)inv[f] * Bp + b]);
+    lam[(size_t)f * Bp + b] = static_cast<double>(Z[(size_t)inv[f] * Bp + (single ? 0 : b)]);
 }
 
 // W[k] = G[perm[k]]: a right-hand side in Jacobian order into pivot order
@@ -908,11 +910,11 @@ template void launch_rows_to_permuted<float>(const int*, int, int, const double*
 template void launch_rows_to_permuted<double>(const int*, int, int, const double*, double*, cudaStream_t);
 
 template <typename T>
-void launch_permuted_to_rows(const int* inv, int dim, int Bp, const T* Z, double* lam, cudaStream_t s) {
-  k_permuted_to_rows<T><<<rows_grid(dim, Bp), dim3(kWarp, kRows), 0, s>>>(inv, dim, Bp, Z, lam);
+void launch_permuted_to_rows(const int* inv, int dim, int Bp, int single, const T* Z, double* lam, cudaStream_t s) {
+  k_permuted_to_rows<T><<<rows_grid(dim, Bp), dim3(kWarp, kRows), 0, s>>>(inv, dim, Bp, single, Z, lam);
 }
-template void launch_permuted_to_rows<float>(const int*, int, int, const float*, double*, cudaStream_t);
-template void launch_permuted_to_rows<double>(const int*, int, int, const double*, double*, cudaStream_t);
+template void launch_permuted_to_rows<float>(const int*, int, int, int, const float*, double*, cudaStream_t);
+template void launch_permuted_to_rows<double>(const int*, int, int, int, const double*, double*, cudaStream_t);
 
 void launch_project_load_gradients(const DevGrid& g, const DevState& st, const double* lam, void* grad_p,
                                    void* grad_q, int is_double, cudaStream_t s) {

@@ -354,7 +354,10 @@ pf_status pf_evaluate(pf_handle h, const double* V, const double* sbus, int32_t 
 pf_status pf_set_profiling(pf_handle h, int32_t enabled);
 pf_status pf_stage_times(pf_handle h, double* times_ms, int64_t* launches);
 /* int64 plan arrays of the engine's factor program: "fe_split", "fe_src",
- * "u_off", "l_off", "cb_off" (same calling convention as pf_plan_array). */
+ * "u_off", "l_off", "cb_off" (same calling convention as pf_plan_array), and
+ * "mismatch_norm_bits": the norms of the last mismatch evaluation as the bits
+ * of doubles, one per column of the batch padded to a multiple of 32 (the
+ * padding repeats the last scenario). */
 pf_status pf_plan_array64(pf_handle h, const char* name, int64_t* out, int64_t capacity, int64_t* len);
 /* Per-scenario static-pivot flags of the last factorization. */
 pf_status pf_singular_flags(pf_handle h, int32_t* out_host, int32_t batch);

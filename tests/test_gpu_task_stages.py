@@ -1,0 +1,91 @@
+"""The subtree-task kernels on the GPU (kernels_task.cuh, kernels_sweep.cuh)
+and what the engine keeps around them."""
+import numpy as np
+import pytest
+
+import cupf
+from cupf import grids as G
+from conftest import gpu_available
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not gpu_available(), reason="needs a CUDA device")]
+
+POLICIES = {p: cupf.ComputePolicy[p] for p in ("FP64", "Mixed", "FP32")}
+
+
+def _grid(buses):
+    return G.make_grid(buses, buses * 3 // 2, buses // 5, seed=1000 + buses)
+
+
+def _newton(g, policy, graph=False, **custom):
+    o = cupf.NewtonOptions(backend=cupf.BackendKind.CUDA, compute=POLICIES[policy])
+    o.use_cuda_graph = graph
+    o.custom.serial_nd = True
+    for k, v in custom.items():
+        setattr(o.custom, k, v)
+    s = cupf.NewtonSolver(o)
+    s.initialize(g.indptr, g.indices, g.data, g.n_bus, g.n_bus, g.pv, g.pq)
+    return s
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("policy", ["FP64", "Mixed", "FP32"])
+@pytest.mark.parametrize("buses", [118, 400, 2000])  # tree launch; tasks with level sweeps; tasks
+def test_padding_columns_of_a_batch_of_one_copy_the_scenario(buses, policy, graph):
+    """The tasks of a single system write one of the 32 columns of the factors;
+    the padding columns of the state still follow the scenario: every column of
+    the padded batch ends with the same mismatch norm."""
+    import torch
+
+    g = _grid(buses)
+    s = _newton(g, policy, graph)
+    tol = 1e-4 if policy == "FP32" else 1e-8
+    S = torch.tensor(g.scenarios(1, seed=buses), device="cuda")
+    _, fm, _ = s.solve_batch_device(S, torch.tensor(g.flat_start(1), device="cuda"),
+                                    config=cupf.NRConfig(tolerance=tol, max_iter=12))
+    norms = s.plan_array64("mismatch_norm_bits").view(np.float64)
+    assert norms.size == 32 and norms[0] <= tol
+    assert (norms == norms[0]).all(), norms
+
+
+def _linear(g, precision, **config):
+    h = cupf.NewtonSolver(cupf.NewtonOptions(backend=cupf.BackendKind.CUDA))
+    h.analyze_host(g.indptr, g.indices, g.n_bus, g.pv, g.pq)
+    rp, ci = h.plan_array("jac_row_ptr"), h.plan_array("jac_col_idx")
+    ls = cupf.LinearSolver(cupf.SolverConfig(precision=int(precision), serial_nd=True, **config))
+    ls.set_data(rp, ci)
+    ls.analyze()
+    return ls, rp, ci
+
+
+def _systems(rp, ci, batch, seed, dtype):
+    """Diagonally dominant values on a pattern, and right-hand sides."""
+    import torch
+
+    rng = np.random.default_rng(seed)
+    vals = rng.standard_normal((batch, ci.size))
+    rows = np.repeat(np.arange(rp.size - 1), np.diff(rp))
+    vals[:, rows == ci] += 8.0
+    return (torch.tensor(vals, dtype=dtype, device="cuda"),
+            torch.tensor(rng.standard_normal((batch, rp.size - 1)), device="cuda"))
+
+
+@pytest.mark.parametrize("precision", [cupf.CustomPrecision.FP64, cupf.CustomPrecision.FP32])
+@pytest.mark.parametrize("buses", [400, 500])  # 300 to 399 fronts: task factors under level sweeps; 400 and more
+def test_batch_of_one_sweeps_equal_the_lane_kernels(buses, precision):
+    """Solve and transpose solve of a batch of one on the factors its tasks
+    left in column 0, against the lane kernels' factors of every column
+    (batch1_schedule = 1): the same bits."""
+    import torch
+
+    g = _grid(buses)
+    dtype = torch.float64 if precision == cupf.CustomPrecision.FP64 else torch.float32
+    out = []
+    for schedule in (0, 1):
+        ls, rp, ci = _linear(g, precision, batch1_schedule=schedule, autotune=False)
+        fronts = ls.plan_array("fp_fsz").size
+        assert (300 <= fronts < 400) if buses == 400 else fronts >= 400
+        A, b = _systems(rp, ci, 1, 5, dtype)
+        ls.setup(1)
+        ls.factorize(A)
+        out.append((ls.solve(b), ls.solve_transpose(b)))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
