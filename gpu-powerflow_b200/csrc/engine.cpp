@@ -81,10 +81,15 @@ struct DBuf {
   T* as() const {
     return static_cast<T*>(p);
   }
+  // Returns once the values are on the device: a copy of pageable memory may
+  // return as soon as they are staged, and a solve runs on streams that the
+  // legacy stream does not order.
   template <typename T>
   void upload(const std::vector<T>& v) {
     reserve(std::max<size_t>(v.size(), 1) * sizeof(T));
-    if (!v.empty()) CUPF_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+    if (v.empty()) return;
+    CUPF_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+    CUPF_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
   }
 };
 

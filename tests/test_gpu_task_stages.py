@@ -47,6 +47,28 @@ def test_padding_columns_of_a_batch_of_one_copy_the_scenario(buses, policy, grap
     assert (norms == norms[0]).all(), norms
 
 
+def test_first_solves_on_a_side_stream_wait_for_their_plans():
+    """What a solve uploads at the first batch of a class is on the device
+    before its kernels run, whatever the default stream has queued."""
+    import torch
+
+    g = _grid(500)
+    busy = torch.randn(4096, 4096, device="cuda")
+    solver, other = _newton(g, "Mixed", autotune=False), torch.cuda.Stream()
+    for batch in (300, 1, 200, 20):  # largest first, then the other classes on its workspace
+        S = torch.tensor(g.scenarios(batch, seed=batch), device="cuda")
+        V0 = torch.tensor(g.flat_start(batch), device="cuda")
+        cfg = cupf.NRConfig(tolerance=1e-8, max_iter=10)
+        want = _newton(g, "Mixed", autotune=False).solve_batch_device(S, V0, config=cfg)[0]
+        torch.cuda.synchronize()
+        for _ in range(8):
+            busy @ busy
+        with torch.cuda.stream(other):
+            got = solver.solve_batch_device(S, V0, config=cfg)[0]
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
+
+
 def _linear(g, precision, **config):
     h = cupf.NewtonSolver(cupf.NewtonOptions(backend=cupf.BackendKind.CUDA))
     h.analyze_host(g.indptr, g.indices, g.n_bus, g.pv, g.pq)
