@@ -37,183 +37,201 @@ struct Arena {
 
 struct Shared {
   const FactorProgram& fp;
-  std::vector<std::vector<int32_t>> kids;  // children, ascending
-  std::vector<double> work;                // of one front
-  std::vector<uint8_t> done;               // factored by an earlier stage
-  std::vector<int32_t> pos;                // position in the task being built, -1 outside it
+  std::vector<std::vector<int32_t>> kids;     // children, ascending
+  std::vector<std::vector<int32_t>> by_size;  // the same, larger fronts first
+  std::vector<double> work;                   // of one front
+  std::vector<int32_t> words;                 // of one front's record, without its external children
+  std::vector<uint8_t> done;                  // factored by an earlier stage
+  std::vector<int32_t> pos;                   // position in the task being built, -1 outside it
+  int ucof(int32_t p) const { return fp.fsz[p] - fp.nc[p]; }
 };
 
 // The fronts below and including the roots that no earlier stage took, children
 // before parents; the larger subtrees first, so that few contribution blocks
-// wait for their parent at a time.
-std::vector<int32_t> task_order(const Shared& sh, const std::vector<int32_t>& roots) {
+// wait for their parent at a time.  Stops once their records exceed max_words.
+std::vector<int32_t> task_order(const Shared& sh, const std::vector<int32_t>& roots, int64_t max_words) {
   std::vector<int32_t> order;
+  std::vector<std::pair<int32_t, size_t>> st;
+  int64_t words = 0;
   for (const int32_t root : roots) {
-    std::vector<std::pair<int32_t, size_t>> st;
-    std::vector<std::vector<int32_t>> todo;
-    auto push = [&](int32_t p) {
-      std::vector<int32_t> c;
-      for (int32_t k : sh.kids[p])
-        if (!sh.done[k]) c.push_back(k);
-      std::stable_sort(c.begin(), c.end(), [&](int32_t a, int32_t b) { return sh.fp.fsz[a] > sh.fp.fsz[b]; });
-      st.push_back({p, 0});
-      todo.push_back(c);
-    };
-    push(root);
+    st.push_back({root, 0});
     while (!st.empty()) {
       auto& [p, k] = st.back();
-      if (k < todo.back().size()) {
-        const int32_t c = todo.back()[k++];
-        push(c);
+      const std::vector<int32_t>& kids = sh.by_size[p];
+      while (k < kids.size() && sh.done[kids[k]]) ++k;
+      if (k < kids.size()) {
+        const int32_t c = kids[k++];
+        st.push_back({c, 0});
       } else {
         order.push_back(p);
+        words += sh.words[p];
+        if (words > max_words) return order;
         st.pop_back();
-        todo.pop_back();
       }
     }
   }
   return order;
 }
 
-// Lists of one front.
-struct FrontLists {
-  std::vector<int32_t> jsrc, jdst, zdst, dst;
-  std::vector<std::vector<int32_t>> pass;  // source arena elements, pass by pass
-  std::vector<int32_t> ext;                // global CB element, elements, arena element
+// Marks a task's fronts with their positions while it is looked at.
+struct Positions {
+  std::vector<int32_t>& pos;
+  const std::vector<int32_t>& order;
+  Positions(std::vector<int32_t>& p, const std::vector<int32_t>& o) : pos(p), order(o) {
+    for (size_t i = 0; i < order.size(); ++i) pos[order[i]] = (int32_t)i;
+  }
+  ~Positions() {
+    for (int32_t p : order) pos[p] = -1;
+  }
 };
 
+// A task of the factorization: its fronts and where their arrays lie in the arena.
 struct TaskBuild {
-  std::vector<int32_t> words;
-  int arena = 0, fronts = 0;
+  std::vector<int32_t> order;
+  std::vector<uint8_t> root;                 // per front
+  std::vector<int> f_at, cb_at;              // dense front; contribution block (-1: none, or it leaves)
+  std::vector<std::vector<int>> src_at;      // per child, its block's arena element (-1: empty)
+  int words = 0, arena = 0;
 };
 
-// The task of the fronts below and including the roots that no earlier stage
-// factored; false when it exceeds the spec's limits.
+// Appends 16-bit lists, padded to whole words.
+void put_halves(std::vector<int32_t>& w, std::vector<uint16_t>& h) {
+  if (h.size() % 2) h.push_back(0);
+  const size_t at = w.size();
+  w.resize(at + h.size() / 2);
+  if (!h.empty()) std::memcpy(w.data() + at, h.data(), h.size() * sizeof(uint16_t));
+}
+
+// Lays out the task of the fronts below and including the roots that no earlier
+// stage factored; false when it exceeds the spec's limits.  Most subtrees are
+// tried and not taken, so this counts the program's words without writing them.
 bool build_task(Shared& sh, const std::vector<int32_t>& roots, const TaskStageSpec& spec, TaskBuild* out) {
   const FactorProgram& fp = sh.fp;
-  const std::vector<int32_t> order = task_order(sh, roots);
-  const auto is_root = [&](int32_t p) { return std::find(roots.begin(), roots.end(), p) != roots.end(); };
+  out->order = task_order(sh, roots, spec.word_cap);
+  const std::vector<int32_t>& order = out->order;
+  int64_t words = 0;
+  for (int32_t p : order) words += sh.words[p];
+  if (words > spec.word_cap) return false;
   const size_t n = order.size();
-  std::vector<int> f_at(n), cb_at(n, -1);
-  std::vector<std::vector<int>> ext_at(n);
-  std::vector<int32_t>& pos = sh.pos;
-  for (size_t i = 0; i < n; ++i) pos[order[i]] = (int32_t)i;
-  struct Reset {
-    std::vector<int32_t>& pos;
-    const std::vector<int32_t>& order;
-    ~Reset() {
-      for (int32_t p : order) pos[p] = -1;
-    }
-  } reset{pos, order};
-  auto cb_size = [&](int32_t p) {
-    const int uc = fp.fsz[p] - fp.nc[p];
-    return uc * (uc + 1);
-  };
+  out->f_at.assign(n, 0);
+  out->cb_at.assign(n, -1);
+  out->src_at.assign(n, {});
+  out->root.assign(n, 0);
+  const Positions mark(sh.pos, order);
+  const std::vector<int32_t>& pos = sh.pos;
+  for (int32_t r : roots) out->root[pos[r]] = 1;
+  auto cb_size = [&](int32_t p) { return sh.ucof(p) * (sh.ucof(p) + 1); };
   Arena ar;
-  auto fetch = [&](size_t i) {  // what the prefetch of front i fills
+  const auto fetch = [&](size_t i) {  // what the prefetch of front i fills
     const int32_t p = order[i];
-    f_at[i] = ar.alloc(fp.fsz[p] * task_front_stride(fp.fsz[p]));
-    for (int32_t c : sh.kids[p])
-      if (pos[c] < 0 && cb_size(c) > 0) ext_at[i].push_back(ar.alloc(cb_size(c)));
+    out->f_at[i] = ar.alloc(fp.fsz[p] * task_front_stride(fp.fsz[p]));
+    for (int32_t c : sh.kids[p]) {
+      const bool ext = pos[c] < 0 && cb_size(c) > 0;
+      out->src_at[i].push_back(ext ? ar.alloc(cb_size(c)) : -1);
+      if (ext) words += 3;
+    }
   };
-  std::vector<std::vector<int>> src_at(n);  // per child of order[i], its block's arena element (-1: empty)
   fetch(0);
   for (size_t i = 0; i < n; ++i) {
     const int32_t p = order[i];
-    size_t e = 0;
-    for (int32_t c : sh.kids[p]) {
-      int at = -1;
-      if (cb_size(c) > 0) at = pos[c] < 0 ? ext_at[i][e++] : cb_at[pos[c]];
-      src_at[i].push_back(at);
-    }
-    for (int at : src_at[i])
+    for (size_t k = 0; k < sh.kids[p].size(); ++k) {
+      int& at = out->src_at[i][k];
+      const int32_t c = sh.kids[p][k];
+      if (pos[c] >= 0) at = out->cb_at[pos[c]];
       if (at >= 0) ar.release(at);
+    }
     if (i + 1 < n) fetch(i + 1);
-    if (!is_root(p) && cb_size(p) > 0) cb_at[i] = ar.alloc(cb_size(p));
-    ar.release(f_at[i]);
+    if (!out->root[i] && cb_size(p) > 0) out->cb_at[i] = ar.alloc(cb_size(p));
+    ar.release(out->f_at[i]);
+    if (ar.peak > spec.arena_cap || ar.peak > 0xffff || words > spec.word_cap) return false;
   }
-  if (ar.peak > spec.arena_cap || ar.peak > 0xffff) return false;
+  out->words = (int)(words + 3) / 4 * 4;
   out->arena = ar.peak;
-  out->fronts = (int)n;
-  // programs
-  std::vector<int32_t>& w = out->words;
-  w.clear();
-  for (size_t i = 0; i < n; ++i) {
-    const int32_t p = order[i];
-    const int fs = fp.fsz[p], nc = fp.nc[p], rs = task_front_stride(fs);
-    FrontLists l;
-    std::vector<uint8_t> set((size_t)fs * (fs + 1), 0);
-    for (int r = 0; r < fs; ++r)
-      for (int32_t a = fp.arow_ptr[fp.front_ptr[p] + r]; a < fp.arow_ptr[fp.front_ptr[p] + r + 1]; ++a) {
-        l.jsrc.push_back(fp.arow_q[a]);
-        l.jdst.push_back(r * rs + fp.arow_col[a]);
-        set[(size_t)r * (fs + 1) + fp.arow_col[a]] = 1;
-      }
-    for (int k = 0; k < nc; ++k) set[(size_t)k * (fs + 1) + fs] = 1;  // the right-hand side rows
-    for (int r = 0; r < fs; ++r)
-      for (int c = 0; c <= fs; ++c)
-        if (!set[(size_t)r * (fs + 1) + c]) l.zdst.push_back(r * rs + c);
-    // child terms per destination, children ascending (the order of every
-    // other assembly of the engine), destinations by falling term count
-    std::vector<std::vector<int32_t>> terms((size_t)fs * (fs + 1));
-    for (size_t ci = 0; ci < sh.kids[p].size(); ++ci) {
-      const int32_t c = sh.kids[p][ci];
-      const int ucc = fp.fsz[c] - fp.nc[c];
-      if (ucc == 0) continue;
-      const int at = src_at[i][ci];
-      if (pos[c] < 0) {
-        l.ext.push_back((int32_t)fp.cb_off[c]);
-        l.ext.push_back(ucc * (ucc + 1));
-        l.ext.push_back(at);
-      }
-      const int32_t* al = fp.asm_local.data() + fp.asm_ptr[c];
-      for (int r = 0; r < ucc; ++r)
-        for (int cc = 0; cc <= ucc; ++cc)
-          terms[(size_t)al[r] * (fs + 1) + (cc < ucc ? al[cc] : fs)].push_back(at + r * (ucc + 1) + cc);
-    }
-    std::vector<int32_t> slots;
-    for (int s = 0; s < fs * (fs + 1); ++s)
-      if (!terms[s].empty()) slots.push_back(s);
-    std::stable_sort(slots.begin(), slots.end(), [&](int32_t a, int32_t b) { return terms[a].size() > terms[b].size(); });
-    const size_t npass = slots.empty() ? 0 : terms[slots[0]].size();
-    l.pass.resize(npass);
-    for (int32_t s : slots) {
-      l.dst.push_back(s / (fs + 1) * rs + s % (fs + 1));
-      for (size_t k = 0; k < terms[s].size(); ++k) l.pass[k].push_back(terms[s][k]);
-    }
+  return out->words <= spec.word_cap;
+}
+
+// Writes the task's program.
+void write_task(Shared& sh, const TaskBuild& t, std::vector<int32_t>& w) {
+  const FactorProgram& fp = sh.fp;
+  const Positions mark(sh.pos, t.order);
+  const size_t begin = w.size();
+  std::vector<int32_t> terms, count, slot_of, dst, pass_at;
+  std::vector<uint16_t> h;
+  std::vector<uint8_t> set;
+  for (size_t i = 0; i < t.order.size(); ++i) {
+    const int32_t p = t.order[i];
+    const int fs = fp.fsz[p], nc = fp.nc[p], rs = task_front_stride(fs), cols = fs + 1;
     const size_t at = w.size();
     w.resize(at + kTaskRecordWords, 0);
-    w[at + kTwShape] = fs | nc << 8 | (is_root(p) ? 1 : 0) << 16;
+    // child terms per destination, children ascending (the order of every
+    // other assembly of the engine), destinations by falling term count
+    terms.assign((size_t)fs * cols, 0);
+    const auto each_term = [&](auto&& f) {
+      for (size_t k = 0; k < sh.kids[p].size(); ++k) {
+        const int32_t c = sh.kids[p][k];
+        const int ucc = sh.ucof(c), from = t.src_at[i][k];
+        const int32_t* al = fp.asm_local.data() + fp.asm_ptr[c];
+        for (int r = 0; r < ucc; ++r)
+          for (int cc = 0; cc <= ucc; ++cc) f(al[r] * cols + (cc < ucc ? al[cc] : fs), from + r * (ucc + 1) + cc);
+      }
+    };
+    int npass = 0;
+    each_term([&](int s, int) { npass = std::max(npass, ++terms[s]); });
+    count.assign(npass + 1, 0);  // destinations with more than k terms
+    for (int32_t n : terms)
+      for (int k = 0; k < n; ++k) ++count[k];
+    slot_of.assign(terms.size(), -1);
+    dst.clear();
+    for (int n = npass; n > 0; --n)
+      for (size_t s = 0; s < terms.size(); ++s)
+        if (terms[s] == n) {
+          slot_of[s] = (int32_t)dst.size();
+          dst.push_back((int32_t)s / cols * rs + (int32_t)s % cols);
+        }
+    w.insert(w.end(), count.begin(), count.begin() + npass);
+    int next = 0;
+    for (size_t k = 0; k < sh.kids[p].size(); ++k) {
+      const int32_t c = sh.kids[p][k];
+      if (sh.pos[c] >= 0 || sh.ucof(c) == 0) continue;
+      w.insert(w.end(), {(int32_t)fp.cb_off[c], sh.ucof(c) * (sh.ucof(c) + 1), t.src_at[i][k]});
+      ++next;
+    }
+    h.clear();
+    set.assign((size_t)fs * cols, 0);
+    int nj = 0;
+    for (int r = 0; r < fs; ++r)
+      for (int32_t a = fp.arow_ptr[fp.front_ptr[p] + r]; a < fp.arow_ptr[fp.front_ptr[p] + r + 1]; ++a, ++nj) {
+        w.push_back(fp.arow_q[a]);
+        h.push_back((uint16_t)(r * rs + fp.arow_col[a]));
+        set[(size_t)r * cols + fp.arow_col[a]] = 1;
+      }
+    for (int k = 0; k < nc; ++k) set[(size_t)k * cols + fs] = 1;  // the right-hand side rows
+    for (int r = 0; r < fs; ++r)
+      for (int c = 0; c < cols; ++c)
+        if (!set[(size_t)r * cols + c]) h.push_back((uint16_t)(r * rs + c));
+    const int nz = (int)h.size() - nj;
+    pass_at.assign(1, (int32_t)w.size());
+    for (int k = 0; k < npass; ++k) pass_at.push_back(pass_at[k] + count[k]);
+    w.resize(pass_at[npass]);
+    std::fill(terms.begin(), terms.end(), 0);
+    each_term([&](int s, int from) {
+      w[pass_at[terms[s]++] + slot_of[s]] = (int32_t)((uint32_t)dst[slot_of[s]] | (uint32_t)from << 16);
+    });
+    w[at + kTwShape] = fs | nc << 8 | t.root[i] << 16;
     w[at + kTwFirst] = fp.first[p];
     w[at + kTwU] = (int32_t)fp.u_off[p];
     w[at + kTwL] = (int32_t)fp.l_off[p];
     w[at + kTwCb] = (int32_t)fp.cb_off[p];
-    w[at + kTwFront] = f_at[i];
-    w[at + kTwCbArena] = cb_at[i];
-    w[at + kTwJ] = (int32_t)(l.jsrc.size() | l.zdst.size() << 16);
-    w[at + kTwPass] = (int32_t)npass;
-    w[at + kTwExt] = (int32_t)(l.ext.size() / 3);
-    for (const auto& q : l.pass) w.push_back((int32_t)q.size());
-    w.insert(w.end(), l.ext.begin(), l.ext.end());
-    w.insert(w.end(), l.jsrc.begin(), l.jsrc.end());
-    for (const auto& q : l.pass)
-      for (size_t k = 0; k < q.size(); ++k) w.push_back((int32_t)((uint32_t)l.dst[k] | (uint32_t)q[k] << 16));
+    w[at + kTwFront] = t.f_at[i];
+    w[at + kTwCbArena] = t.cb_at[i];
+    w[at + kTwJ] = (int32_t)((uint32_t)nj | (uint32_t)nz << 16);
+    w[at + kTwPass] = npass;
+    w[at + kTwExt] = next;
     w[at + kTwHalf] = (int32_t)(w.size() - at);
-    std::vector<uint16_t> h;
-    auto put = [&](const std::vector<int32_t>& v) {
-      for (int32_t x : v) h.push_back((uint16_t)x);
-    };
-    put(l.jdst);
-    put(l.zdst);
-    if (h.size() % 2) h.push_back(0);
-    const size_t hw = w.size();
-    w.resize(hw + h.size() / 2);
-    if (!h.empty()) std::memcpy(w.data() + hw, h.data(), h.size() * sizeof(uint16_t));
+    put_halves(w, h);
     w[at + kTwNext] = (int32_t)(w.size() - at);
-    if ((int)w.size() > spec.word_cap) return false;
   }
-  while (w.size() % 4) w.push_back(0);
-  return (int)w.size() <= spec.word_cap;
+  while ((w.size() - begin) % 4) w.push_back(0);
 }
 
 // Cuts the tree into stages of tasks.  out marks the fronts to leave out
@@ -315,144 +333,183 @@ void cut_tree(Shared& sh, std::vector<uint8_t>& out, const std::vector<TaskStage
 bool link_tree(const FactorProgram& fp, Shared* sh) {
   sh->kids.resize(fp.P);
   sh->work.resize(fp.P);
+  sh->words.resize(fp.P);
   sh->done.assign(fp.P, 0);
   for (int32_t p = 0; p < fp.P; ++p) {
     const int32_t par = fp.parent_panel[p];
     if (par >= 0 && par <= p) return false;
     if (par >= 0) sh->kids[par].push_back(p);
   }
+  sh->by_size = sh->kids;
+  for (auto& k : sh->by_size)
+    std::stable_sort(k.begin(), k.end(), [&](int32_t a, int32_t b) { return fp.fsz[a] > fp.fsz[b]; });
   return true;
 }
 
+// A task of the sweeps: its fronts, and where their update vectors lie in the arena.
 struct SweepBuild {
-  std::vector<int32_t> words;
-  int fronts = 0, ext_rows = 0, local = 0, arena = 0, rows = 0, max_u = 0, max_l = 0;
+  std::vector<int32_t> order, ext_rows;  // ext_rows: the roots' contribution rows
+  std::vector<int> tv_at;                // update vector (-1: none, or it leaves)
+  std::vector<std::vector<int>> src_at;  // per child, its vector's arena element (-1: empty)
+  int local = 0, words = 0, arena = 0, rows = 0, max_u = 0, max_l = 0;
 };
 
-bool build_sweep_task(Shared& sh, const std::vector<int32_t>& roots, const TaskStageSpec& spec, const std::vector<int64_t>& tv_off,
-                      const std::vector<int32_t>& level_counts, SweepBuild* out) {
+// As build_task; the local numbers are the task's pivots, then ext_rows.
+bool build_sweep_task(Shared& sh, const std::vector<int32_t>& roots, const TaskStageSpec& spec, SweepBuild* out) {
   const FactorProgram& fp = sh.fp;
-  const std::vector<int32_t> order = task_order(sh, roots);
+  out->order = task_order(sh, roots, spec.word_cap);
+  const std::vector<int32_t>& order = out->order;
   const size_t n = order.size();
-  const auto ucof = [&](int32_t p) { return fp.fsz[p] - fp.nc[p]; };
-  const auto is_root = [&](int32_t p) { return std::find(roots.begin(), roots.end(), p) != roots.end(); };
-  // local numbers: the task's pivots, then the roots' contribution rows
+  int64_t words = (int64_t)n;
   int npiv = 0;
-  for (int32_t p : order) npiv += fp.nc[p];
-  std::vector<int32_t> ext_rows;
-  for (int32_t r : roots)
-    ext_rows.insert(ext_rows.end(), fp.front_rows.begin() + fp.front_ptr[r] + fp.nc[r],
-                    fp.front_rows.begin() + fp.front_ptr[r + 1]);
-  std::sort(ext_rows.begin(), ext_rows.end());
-  ext_rows.erase(std::unique(ext_rows.begin(), ext_rows.end()), ext_rows.end());
-  out->local = npiv + (int)ext_rows.size();
-  out->ext_rows = (int)ext_rows.size();
-  out->fronts = (int)n;
-  if (out->local > spec.arena_cap || out->local > 0xffff) return false;
-  std::vector<int32_t>& pos = sh.pos;
-  for (size_t i = 0; i < n; ++i) pos[order[i]] = (int32_t)i;
-  struct Reset {
-    std::vector<int32_t>& pos;
-    const std::vector<int32_t>& order;
-    ~Reset() {
-      for (int32_t p : order) pos[p] = -1;
-    }
-  } reset{pos, order};
-  std::vector<int> lp(n), tv_at(n, -1);
-  std::vector<std::pair<int32_t, int>> local;  // global pivot row -> local number
-  int at = 0;
-  for (size_t i = 0; i < n; ++i) {
-    const int32_t p = order[i];
-    lp[i] = at;
-    for (int k = 0; k < fp.nc[p]; ++k) local.push_back({fp.first[p] + k, at++});
+  *out = SweepBuild{std::move(out->order), {}, {}, {}};
+  for (int32_t p : order) {
+    const int fs = fp.fsz[p], nc = fp.nc[p], uc = fs - nc;
+    words += sh.words[p];
+    npiv += nc;
+    out->rows = std::max(out->rows, fs);
+    out->max_u = std::max(out->max_u, nc * fs);
+    out->max_l = std::max(out->max_l, uc * nc);
   }
-  for (int32_t row : ext_rows) local.push_back({row, at++});
-  std::sort(local.begin(), local.end());
-  const auto number = [&](int32_t row) {
-    const auto it = std::lower_bound(local.begin(), local.end(), std::make_pair(row, -1));
-    return it != local.end() && it->first == row ? it->second : -1;
-  };
+  if (words > spec.word_cap) return false;
+  if (out->max_u > spec.factor_cap || 64 + out->max_l > spec.factor_cap || out->rows > spec.factor_cap) return false;
+  std::vector<int32_t>& ext = out->ext_rows;
+  for (int32_t r : roots)
+    ext.insert(ext.end(), fp.front_rows.begin() + fp.front_ptr[r] + fp.nc[r],
+               fp.front_rows.begin() + fp.front_ptr[r + 1]);
+  std::sort(ext.begin(), ext.end());
+  ext.erase(std::unique(ext.begin(), ext.end()), ext.end());
+  words += (int64_t)ext.size();
+  out->local = npiv + (int)ext.size();
+  if (out->local > spec.arena_cap || out->local > 0xffff) return false;
+  const Positions mark(sh.pos, order);
+  const std::vector<int32_t>& pos = sh.pos;
+  std::vector<uint8_t> root(n, 0);
+  for (int32_t r : roots) root[pos[r]] = 1;
   // update vectors in the arena: a front's external children are fetched with
   // its factors, sweep_ring - 1 fronts ahead
   Arena ar;
-  std::vector<std::vector<int>> ext_at(n), src_at(n);
+  out->tv_at.assign(n, -1);
+  out->src_at.assign(n, {});
   const auto fetch = [&](size_t i) {
-    for (int32_t c : sh.kids[order[i]])
-      if (pos[c] < 0 && ucof(c) > 0) ext_at[i].push_back(ar.alloc(ucof(c)));
+    for (int32_t c : sh.kids[order[i]]) {
+      const bool e = pos[c] < 0 && sh.ucof(c) > 0;
+      out->src_at[i].push_back(e ? ar.alloc(sh.ucof(c)) : -1);
+      if (e) words += 3;
+    }
   };
   const size_t ahead = (size_t)sweep_ring(spec.warps) - 1;
   for (size_t i = 0; i < std::min(ahead, n); ++i) fetch(i);
   for (size_t i = 0; i < n; ++i) {
     const int32_t p = order[i];
-    size_t e = 0;
-    for (int32_t c : sh.kids[p]) src_at[i].push_back(ucof(c) == 0 ? -1 : pos[c] < 0 ? ext_at[i][e++] : tv_at[pos[c]]);
-    for (int a : src_at[i])
-      if (a >= 0) ar.release(a);
+    for (size_t k = 0; k < sh.kids[p].size(); ++k) {
+      int& at = out->src_at[i][k];
+      const int32_t c = sh.kids[p][k];
+      if (pos[c] >= 0) at = out->tv_at[pos[c]];
+      if (at >= 0) ar.release(at);
+    }
     if (i + ahead < n) fetch(i + ahead);
-    if (!is_root(p) && ucof(p) > 0) tv_at[i] = ar.alloc(ucof(p));
+    if (!root[i] && sh.ucof(p) > 0) out->tv_at[i] = ar.alloc(sh.ucof(p));
+    if (ar.peak > spec.arena_cap || ar.peak > 0xffff || words > spec.word_cap) return false;
   }
+  out->words = (int)(words + 3) / 4 * 4;
   out->arena = ar.peak;
-  if (ar.peak > spec.arena_cap || ar.peak > 0xffff) return false;
-  std::vector<int32_t>& w = out->words;
-  w.assign(n, 0);
-  w.insert(w.end(), ext_rows.begin(), ext_rows.end());
+  return out->words <= spec.word_cap;
+}
+
+// Writes the task's program; number: scratch, -1 for every row.  False when a
+// front's row is neither a pivot of the task nor a row of its roots.
+bool write_sweep_task(Shared& sh, const SweepBuild& t, const std::vector<int64_t>& tv_off,
+                      const std::vector<int32_t>& level_counts, std::vector<int32_t>& number,
+                      std::vector<int32_t>& w) {
+  const FactorProgram& fp = sh.fp;
+  const Positions mark(sh.pos, t.order);
+  const size_t begin = w.size(), n = t.order.size();
+  std::vector<int> lp(n);
+  int at = 0;
   for (size_t i = 0; i < n; ++i) {
-    const int32_t p = order[i];
+    const int32_t p = t.order[i];
+    lp[i] = at;
+    for (int k = 0; k < fp.nc[p]; ++k) number[fp.first[p] + k] = at++;
+  }
+  for (int32_t row : t.ext_rows) number[row] = at++;
+  bool ok = true;
+  w.resize(begin + n, 0);
+  w.insert(w.end(), t.ext_rows.begin(), t.ext_rows.end());
+  std::vector<int32_t> terms, count, slot_of, pass_at;
+  std::vector<uint16_t> h, rows;
+  for (size_t i = 0; i < n; ++i) {
+    const int32_t p = t.order[i];
     const int fs = fp.fsz[p], nc = fp.nc[p], uc = fs - nc;
     const size_t r = w.size();
-    w[i] = (int32_t)r;
-    out->rows = std::max(out->rows, fs);
-    out->max_u = std::max(out->max_u, nc * fs);
-    out->max_l = std::max(out->max_l, uc * nc);
-    if (nc * fs > spec.factor_cap || 64 + uc * nc > spec.factor_cap || fs > spec.factor_cap) return false;
-    std::vector<std::vector<int32_t>> terms(fs);
-    std::vector<int32_t> ext;
-    for (size_t ci = 0; ci < sh.kids[p].size(); ++ci) {
-      const int32_t c = sh.kids[p][ci];
-      if (ucof(c) == 0) continue;
-      if (pos[c] < 0) ext.insert(ext.end(), {(int32_t)tv_off[c], ucof(c), src_at[i][ci]});
-      const int32_t* al = fp.asm_local.data() + fp.asm_ptr[c];
-      for (int q = 0; q < ucof(c); ++q) terms[al[q]].push_back(src_at[i][ci] + q);
-    }
-    std::vector<int32_t> rows;
-    for (int q = 0; q < fs; ++q) rows.push_back(q);  // (rows without terms come last and start at zero)
-    std::stable_sort(rows.begin(), rows.end(), [&](int32_t a, int32_t b) { return terms[a].size() > terms[b].size(); });
-    const size_t npass = terms[rows[0]].size();
-    std::vector<std::vector<int32_t>> pass(npass);
-    for (int32_t q : rows)
-      for (size_t k = 0; k < terms[q].size(); ++k) pass[k].push_back(terms[q][k]);
+    w[begin + i] = (int32_t)(r - begin);
     w.resize(r + kSweepRecordWords, 0);
+    // child terms per row, children ascending; rows by falling term count
+    // (rows without terms come last and start at zero)
+    terms.assign(fs, 0);
+    int npass = 0;
+    for (const int32_t c : sh.kids[p]) {
+      const int32_t* al = fp.asm_local.data() + fp.asm_ptr[c];
+      for (int q = 0; q < sh.ucof(c); ++q) npass = std::max(npass, ++terms[al[q]]);
+    }
+    count.assign(npass + 1, 0);  // rows with more than k terms
+    for (int32_t m : terms)
+      for (int k = 0; k < m; ++k) ++count[k];
+    slot_of.assign(fs, 0);
+    rows.clear();
+    for (int m = npass; m >= 0; --m)
+      for (int q = 0; q < fs; ++q)
+        if (terms[q] == m) {
+          slot_of[q] = (int32_t)rows.size();
+          rows.push_back((uint16_t)q);
+        }
+    w.insert(w.end(), count.begin(), count.begin() + npass);
+    int next = 0;
+    for (size_t k = 0; k < sh.kids[p].size(); ++k) {
+      const int32_t c = sh.kids[p][k];
+      if (sh.pos[c] >= 0 || sh.ucof(c) == 0) continue;
+      w.insert(w.end(), {(int32_t)tv_off[c], sh.ucof(c), t.src_at[i][k]});
+      ++next;
+    }
     w[r + kSwShape] = fs | nc << 16;
     w[r + kSwFirst] = fp.first[p];
     w[r + kSwU] = (int32_t)fp.u_off[p];
     w[r + kSwL] = (int32_t)fp.l_off[p];
     w[r + kSwLocal] = lp[i];
     w[r + kSwTv] = (int32_t)tv_off[p];
-    w[r + kSwTvArena] = tv_at[i];
-    w[r + kSwPass] = (int32_t)npass;
-    w[r + kSwExt] = (int32_t)(ext.size() / 3);
+    w[r + kSwTvArena] = t.tv_at[i];
+    w[r + kSwPass] = npass;
+    w[r + kSwExt] = next;
     w[r + kSwLevel] = level_counts[p];
-    for (const auto& q : pass) w.push_back((int32_t)q.size());
-    w.insert(w.end(), ext.begin(), ext.end());
     w[r + kSwLists] = (int32_t)(w.size() - r);
-    std::vector<uint16_t> h;
+    h.clear();
     for (int j = 0; j < uc; ++j) {
-      const int num = number(fp.front_rows[fp.front_ptr[p] + nc + j]);
-      if (num < 0) return false;
+      const int32_t num = number[fp.front_rows[fp.front_ptr[p] + nc + j]];
+      ok = ok && num >= 0;
       h.push_back((uint16_t)num);
     }
-    for (int32_t q : rows) h.push_back((uint16_t)q);
-    for (const auto& q : pass)
-      for (int32_t s : q) h.push_back((uint16_t)s);
-    if (h.size() % 2) h.push_back(0);
-    const size_t hw = w.size();
-    w.resize(hw + h.size() / 2);
-    if (!h.empty()) std::memcpy(w.data() + hw, h.data(), h.size() * sizeof(uint16_t));
-    if ((int)w.size() > spec.word_cap) return false;
+    h.insert(h.end(), rows.begin(), rows.end());
+    pass_at.assign(1, (int32_t)h.size());
+    for (int k = 0; k < npass; ++k) pass_at.push_back(pass_at[k] + count[k]);
+    h.resize(pass_at[npass]);
+    std::fill(terms.begin(), terms.end(), 0);
+    for (size_t k = 0; k < sh.kids[p].size(); ++k) {
+      const int32_t c = sh.kids[p][k];
+      const int32_t* al = fp.asm_local.data() + fp.asm_ptr[c];
+      for (int q = 0; q < sh.ucof(c); ++q)
+        h[pass_at[terms[al[q]]++] + slot_of[al[q]]] = (uint16_t)(t.src_at[i][k] + q);
+    }
+    put_halves(w, h);
   }
-  while (w.size() % 4) w.push_back(0);
-  return (int)w.size() <= spec.word_cap;
+  while ((w.size() - begin) % 4) w.push_back(0);
+  for (int32_t p : t.order)
+    for (int k = 0; k < fp.nc[p]; ++k) number[fp.first[p] + k] = -1;
+  for (int32_t row : t.ext_rows) number[row] = -1;
+  return ok;
 }
+
+// Words of the halves of a record's lists.
+int half_words(int64_t halves) { return (int)((halves + 1) / 2); }
 
 }  // namespace
 
@@ -511,17 +568,36 @@ TaskPlan build_task_plan(const FactorProgram& fp, int front_limit, const std::ve
   // element offsets and list lengths must fit the program's fields
   if (fp.u_total > INT32_MAX || fp.l_total > INT32_MAX || fp.cb_total > INT32_MAX || specs.empty()) return none;
   front_limit = std::min(front_limit, 128);
-  Shared sh{fp, {}, {}, {}, std::vector<int32_t>(fp.P, -1)};
+  Shared sh{fp, {}, {}, {}, {}, {}, std::vector<int32_t>(fp.P, -1)};
   if (!link_tree(fp, &sh)) return none;
   std::vector<uint8_t> out(fp.P, 0);  // left to the level launches
+  std::vector<int32_t> scratch;
   for (int32_t p = 0; p < fp.P; ++p) {
     const double fs = fp.fsz[p], nc = fp.nc[p], uc = fs - nc;
     sh.work[p] = 60 + fs * (fs + 1) + uc * (uc + 1) * (2 + nc) / 2;
     for (int32_t fr = fp.front_ptr[p]; fr < fp.front_ptr[p + 1]; ++fr)
       for (int32_t a = fp.arow_ptr[fr] + 1; a < fp.arow_ptr[fr + 1]; ++a)
         if (fp.arow_col[a] == fp.arow_col[a - 1]) return none;
-    if (fp.fsz[p] >= front_limit)
+    if (fp.fsz[p] >= front_limit) {
       for (int32_t q = p; q >= 0 && !out[q]; q = fp.parent_panel[q]) out[q] = 1;
+      continue;
+    }
+    // words of its record
+    std::vector<int32_t>& count = scratch;
+    count.assign((size_t)fp.fsz[p] * (fp.fsz[p] + 1), 0);
+    int64_t nj = fp.arow_ptr[fp.front_ptr[p + 1]] - fp.arow_ptr[fp.front_ptr[p]], terms = 0;
+    int npass = 0;
+    for (int32_t c : sh.kids[p]) {
+      const int ucc = sh.ucof(c);
+      const int32_t* al = fp.asm_local.data() + fp.asm_ptr[c];
+      for (int r = 0; r < ucc; ++r)
+        for (int k = 0; k <= ucc; ++k)
+          npass = std::max(npass, ++count[(size_t)al[r] * (fp.fsz[p] + 1) + (k < ucc ? al[k] : fp.fsz[p])]);
+      terms += (int64_t)ucc * (ucc + 1);
+    }
+    // (16-bit lists: every element but the right-hand side rows')
+    const int64_t words = kTaskRecordWords + npass + nj + terms + half_words((int64_t)count.size() - fp.nc[p]);
+    sh.words[p] = (int32_t)std::min<int64_t>(words, INT32_MAX);
   }
   TaskPlan tp;
   cut_tree<TaskBuild>(
@@ -536,9 +612,9 @@ TaskPlan build_task_plan(const FactorProgram& fp, int front_limit, const std::ve
         st.lanes = spec.lanes;
         st.pack = spec.pack;
         for (const TaskBuild& t : tasks) {
-          tp.meta.insert(tp.meta.end(), {(int32_t)tp.words.size(), (int32_t)t.words.size(), t.fronts, 0});
-          tp.words.insert(tp.words.end(), t.words.begin(), t.words.end());
-          st.max_words = std::max(st.max_words, (int)t.words.size());
+          tp.meta.insert(tp.meta.end(), {(int32_t)tp.words.size(), t.words, (int32_t)t.order.size(), 0});
+          write_task(sh, t, tp.words);
+          st.max_words = std::max(st.max_words, t.words);
           st.max_arena = std::max(st.max_arena, t.arena);
         }
         tp.stages.push_back(st);
@@ -550,13 +626,24 @@ TaskPlan build_task_plan(const FactorProgram& fp, int front_limit, const std::ve
 SweepPlan build_sweep_plan(const FactorProgram& fp, const std::vector<TaskStageSpec>& specs,
                            const std::vector<int32_t>& level_counts) {
   if (fp.u_total > INT32_MAX || fp.l_total > INT32_MAX || specs.empty()) return {};
-  Shared sh{fp, {}, {}, {}, std::vector<int32_t>(fp.P, -1)};
+  Shared sh{fp, {}, {}, {}, {}, {}, std::vector<int32_t>(fp.P, -1)};
   if (!link_tree(fp, &sh)) return {};
   std::vector<int64_t> tv(fp.P + 1, 0);
+  std::vector<int32_t> count, number(fp.dim, -1);
+  bool ok = true;
   for (int32_t p = 0; p < fp.P; ++p) {
     tv[p + 1] = tv[p] + (fp.fsz[p] - fp.nc[p]);
     sh.work[p] = 30 + fp.nc[p] * fp.fsz[p];
     if (fp.fsz[p] > 0xffff || fp.nc[p] > 8) return {};
+    int64_t terms = 0;
+    int npass = 0;
+    count.assign(fp.fsz[p], 0);
+    for (int32_t c : sh.kids[p]) {
+      const int32_t* al = fp.asm_local.data() + fp.asm_ptr[c];
+      for (int q = 0; q < sh.ucof(c); ++q) npass = std::max(npass, ++count[al[q]]);
+      terms += sh.ucof(c);
+    }
+    sh.words[p] = kSweepRecordWords + npass + half_words(sh.ucof(p) + fp.fsz[p] + terms);
   }
   if (tv[fp.P] > INT32_MAX) return {};
   std::vector<uint8_t> out(fp.P, 0);
@@ -564,7 +651,7 @@ SweepPlan build_sweep_plan(const FactorProgram& fp, const std::vector<TaskStageS
   cut_tree<SweepBuild>(
       sh, out, specs,
       [&](const std::vector<int32_t>& roots, const TaskStageSpec& spec, SweepBuild* t) {
-        return build_sweep_task(sh, roots, spec, tv, level_counts, t);
+        return build_sweep_task(sh, roots, spec, t);
       },
       [&](const std::vector<SweepBuild>& tasks, const TaskStageSpec& spec) {
         SweepTaskStage st;
@@ -574,9 +661,10 @@ SweepPlan build_sweep_plan(const FactorProgram& fp, const std::vector<TaskStageS
         st.lanes = spec.lanes;
         st.pack = spec.pack;
         for (const SweepBuild& t : tasks) {
-          sp.meta.insert(sp.meta.end(), {(int32_t)sp.words.size(), (int32_t)t.words.size(), t.fronts, t.ext_rows});
-          sp.words.insert(sp.words.end(), t.words.begin(), t.words.end());
-          st.max_words = std::max(st.max_words, (int)t.words.size());
+          sp.meta.insert(sp.meta.end(), {(int32_t)sp.words.size(), t.words, (int32_t)t.order.size(),
+                                         (int32_t)t.ext_rows.size()});
+          ok = write_sweep_task(sh, t, tv, level_counts, number, sp.words) && ok;
+          st.max_words = std::max(st.max_words, t.words);
           st.max_local = std::max(st.max_local, t.local);
           st.max_arena = std::max(st.max_arena, t.arena);
           st.max_rows = std::max(st.max_rows, t.rows);
@@ -587,6 +675,7 @@ SweepPlan build_sweep_plan(const FactorProgram& fp, const std::vector<TaskStageS
       });
   for (uint8_t d : sh.done)
     if (!d) return {};  // a front too large for a task
+  if (!ok) return {};
   return sp;
 }
 
