@@ -25,7 +25,6 @@
 
 #include "kernels.hpp"
 #include "static_scratch.hpp"
-#include "task_plan.hpp"
 
 namespace cupf_b200 {
 
@@ -100,16 +99,18 @@ std::vector<long long> to_ll(const std::vector<T>& v) {
 
 }  // namespace
 
-// Subtree tasks of the factorization and the sweeps (task_plan.hpp), one set
-// per class of batch size, and the level launches of the fronts no
-// factorization task covers, with launch records and source lists of their
-// own.
+// Subtree tasks of the factorization (task_plan.hpp) on the device, one set per
+// class of batch size, and the level launches of the fronts no task covers,
+// with launch records and source lists of their own.
 struct Engine::TaskSet {
   TaskPlan tasks;
-  SweepPlan sweeps;  // empty: a front is too large, and the sweeps run level by level
-  DBuf task_meta, task_words, sweep_meta, sweep_words, rest_meta, rest_src, rest_dst;
+  DBuf meta, words, rest_meta, rest_src, rest_dst;
   std::vector<LevelLaunch> rest;
-  bool uploaded = false;
+};
+// The sweeps' tasks (plan empty: a front is too large, and the sweeps run level by level).
+struct Engine::SweepSet {
+  SweepPlan plan;
+  DBuf meta, words;
 };
 
 struct Engine::Impl {
@@ -120,8 +121,16 @@ struct Engine::Impl {
   DBuf fsz, nc, first, front_ptr, front_rows, u_off, l_off, cb_off, tv_off, arow_ptr, arow_q, arow_col, crow_ptr,
       crow_child, crow_r, crow_src, crow_dst, asm_ptr, asm_local, perm, iperm, row_iperm, col_perm, level_fronts, fe_split, fe_dst, fe_src, front_meta;
   std::vector<LevelLaunch> levels;
-  std::map<int, std::unique_ptr<TaskSet>> task_sets;
-  TaskSet* ts = nullptr;  // of the current batch
+  std::map<int, std::unique_ptr<TaskSet>> task_sets;    // by class
+  std::map<int, std::unique_ptr<SweepSet>> sweep_sets;  // by sweep_class(class)
+  TaskSet* ts = nullptr;                                // of the current batch (null: the level launches)
+  SweepSet* sweeps = nullptr;
+  void clear_tasks() {
+    ts = nullptr;
+    sweeps = nullptr;
+    task_sets.clear();
+    sweep_sets.clear();
+  }
   int graph_lanes = 0;    // tasks' scenarios of the captured solve
   int single_batch() const { return B == 1 ? 1 : 0; }
   int task_lanes() const { return B == 1 ? 1 : Bp; }  // scenarios the tasks cover (padding included)
@@ -239,15 +248,21 @@ bool Engine::tf32_factors() const { return cfg_.factor_precision == kFactorTF32 
 
 bool Engine::single_system() const { return cfg_.batch1_schedule == 0 && d_->B == 1; }
 
+// Small trees are a few short levels, and the stages' launches cost as much
+// as the levels': per graph-mode iteration 94 against 113 us by levels and
+// by tasks with 100 buses (about 75 fronts) x 64, 127 against 126 us with
+// 300 buses (about 250 fronts), 220 against 185 us with 1,000.
+constexpr int kTaskFronts = 300;
+// Small trees sweep level by level: factorize + solve + transpose solve with
+// 300 buses (about 250 fronts) x 20 takes 321 us by levels and 349 us by
+// tasks, 610 and 696 us x 1,500 in FP64; 500 buses (420 fronts) x 200 515 and
+// 448 us, 800 buses x 300 635 and 532 us.
+constexpr int kSweepTaskFronts = 400;
+
 bool Engine::use_tasks() const {
-  if (d_->ts->tasks.stages.empty() || (d_->B == 1 && cfg_.batch1_schedule == 1)) return false;
-  // Small trees are a few short levels, and the stages' launches cost as much
-  // as the levels': per graph-mode iteration 94 against 113 us by levels and
-  // by tasks with 100 buses (about 75 fronts) x 64, 127 against 126 us with
-  // 300 buses (about 250 fronts), 220 against 185 us with 1,000.  For a single
-  // system the other way is one launch over the whole tree.
-  if (single_system() && !d_->ts->rest.empty()) return false;
-  return fp_.P >= 300;
+  if (!d_->ts || d_->ts->tasks.stages.empty() || (d_->B == 1 && cfg_.batch1_schedule == 1)) return false;
+  // for a single system the other way is one launch over the whole tree
+  return !(single_system() && !d_->ts->rest.empty());
 }
 
 // The single-system factorization as one tree launch: batch 1, no
@@ -428,58 +443,80 @@ std::vector<LevelLaunch> Engine::level_launches(const std::vector<std::vector<in
 // option sends to another kernel (the any-size tier, the tensor cores) stay
 // with the level launches of the factorization, as do fronts too large for a
 // task.
-Engine::TaskSet& Engine::task_set(int cls) const {
-  auto& d = *d_;
-  auto& slot = d.task_sets[cls];
-  if (slot) return *slot;
-  slot = std::make_unique<TaskSet>();
+TaskPlan Engine::task_plan(int cls) const {
   int limit = std::min(cfg_.wide_min_front > 0 ? cfg_.wide_min_front : kWideFrontRows, kWideFrontRows);
   if (tf32_factors())
     limit = std::min(limit, cfg_.tc_min_front > 0 ? cfg_.tc_min_front
                             : cfg_.autotune       ? kTcSmallestMinFront
                                                   : kTcDefaultMinFront);
-  slot->tasks = build_task_plan(fp_, limit, factor_task_specs(cls, factor_is_double() ? 8 : 4));
+  return build_task_plan(fp_, limit, factor_task_specs(cls, factor_is_double() ? 8 : 4));
+}
+
+SweepPlan Engine::sweep_plan(int cls) const {
   std::vector<std::vector<int32_t>> by_level(fp_.num_levels);
   for (int32_t L = 0; L < fp_.num_levels; ++L)
     by_level[L].assign(fp_.level_fronts.begin() + fp_.level_ptr[L], fp_.level_fronts.begin() + fp_.level_ptr[L + 1]);
   std::vector<int32_t> counts(fp_.P, 0);
   for (const LevelLaunch& lv : level_launches(by_level))
     for (int32_t q = lv.begin; q < lv.begin + lv.count; ++q) counts[fp_.level_fronts[q]] = lv.count;
-  slot->sweeps = build_sweep_plan(fp_, sweep_task_specs(cls), counts);
-  return *slot;
+  return build_sweep_plan(fp_, sweep_task_specs(cls), counts);
 }
 
-// Makes the current batch's task set the one in use (uploading it at its
-// first batch).
+// Builds and uploads the plans of every class that a batch of up to B systems
+// can have, so that a smaller batch on this workspace allocates and plans
+// nothing; trees below the thresholds, which use neither, get none.  All four
+// classes take about as long as the symbolic analysis (2,000 buses: 15 ms).
+void Engine::prepare_tasks(int32_t B) {
+  auto& d = *d_;
+  std::vector<int> classes{task_class(fp_.P, 1)};
+  if (B > 1)  // (the classes of larger batches follow one another)
+    for (int c = task_class(fp_.P, 2); c <= task_class(fp_.P, B); ++c) classes.push_back(c);
+  for (int cls : classes) {
+    if (fp_.P >= kTaskFronts && !d.task_sets.count(cls)) {
+      auto ts = std::make_unique<TaskSet>();
+      ts->tasks = task_plan(cls);
+      ts->meta.upload(ts->tasks.meta);
+      ts->words.upload(ts->tasks.words);
+      if (!ts->tasks.stages.empty()) {
+        // the fronts no task covers, level by level
+        std::vector<std::vector<int32_t>> by_level(fp_.num_levels);
+        std::vector<int32_t> order, qof(fp_.P), meta;
+        for (int32_t L = 0; L < fp_.num_levels; ++L)
+          for (int32_t q = fp_.level_ptr[L]; q < fp_.level_ptr[L + 1]; ++q) {
+            const int32_t p = fp_.level_fronts[q];
+            qof[p] = q;
+            if (!ts->tasks.covered[p]) by_level[L].push_back(p);
+          }
+        ts->rest = level_launches(by_level);
+        for (const auto& lv : by_level) order.insert(order.end(), lv.begin(), lv.end());
+        for (int32_t p : order)
+          meta.insert(meta.end(), fp_.front_meta.begin() + (size_t)qof[p] * kFrontMetaInts,
+                      fp_.front_meta.begin() + (size_t)(qof[p] + 1) * kFrontMetaInts);
+        ts->rest_meta.upload(meta);
+        pad_lists(ts->rest, order, ts->rest_src, ts->rest_dst);
+      }
+      d.task_sets[cls] = std::move(ts);
+      assign_tiers(tc_min_);
+    }
+    const int sc = sweep_class(cls);
+    if (fp_.P >= kSweepTaskFronts && !d.sweep_sets.count(sc)) {
+      auto ss = std::make_unique<SweepSet>();
+      ss->plan = sweep_plan(cls);
+      ss->meta.upload(ss->plan.meta);
+      ss->words.upload(ss->plan.words);
+      d.sweep_sets[sc] = std::move(ss);
+    }
+  }
+}
+
+// Makes the current batch's plans the ones in use.
 void Engine::select_tasks() {
   auto& d = *d_;
-  TaskSet& ts = task_set(task_class(fp_.P, d.B));
-  d.ts = &ts;
-  if (ts.uploaded) return;
-  ts.task_meta.upload(ts.tasks.meta);
-  ts.task_words.upload(ts.tasks.words);
-  ts.sweep_meta.upload(ts.sweeps.meta);
-  ts.sweep_words.upload(ts.sweeps.words);
-  if (!ts.tasks.stages.empty()) {
-    // the fronts no task covers, level by level
-    std::vector<std::vector<int32_t>> by_level(fp_.num_levels);
-    std::vector<int32_t> order, qof(fp_.P), meta;
-    for (int32_t L = 0; L < fp_.num_levels; ++L)
-      for (int32_t q = fp_.level_ptr[L]; q < fp_.level_ptr[L + 1]; ++q) {
-        const int32_t p = fp_.level_fronts[q];
-        qof[p] = q;
-        if (!ts.tasks.covered[p]) by_level[L].push_back(p);
-      }
-    ts.rest = level_launches(by_level);
-    for (const auto& lv : by_level) order.insert(order.end(), lv.begin(), lv.end());
-    for (int32_t p : order)
-      meta.insert(meta.end(), fp_.front_meta.begin() + (size_t)qof[p] * kFrontMetaInts,
-                  fp_.front_meta.begin() + (size_t)(qof[p] + 1) * kFrontMetaInts);
-    ts.rest_meta.upload(meta);
-    pad_lists(ts.rest, order, ts.rest_src, ts.rest_dst);
-    assign_tiers(tc_min_);
-  }
-  ts.uploaded = true;
+  const int cls = task_class(fp_.P, d.B);
+  const auto ts = d.task_sets.find(cls);
+  const auto ss = d.sweep_sets.find(sweep_class(cls));
+  d.ts = ts == d.task_sets.end() ? nullptr : ts->second.get();
+  d.sweeps = ss == d.sweep_sets.end() ? nullptr : ss->second.get();
 }
 
 // Source lists in launch order, each padded to its launch's longest.
@@ -562,8 +599,7 @@ void Engine::upload_plan() {
   for (int32_t L = 0; L < fp_.num_levels; ++L)
     by_level[L].assign(fp_.level_fronts.begin() + fp_.level_ptr[L], fp_.level_fronts.begin() + fp_.level_ptr[L + 1]);
   d.levels = level_launches(by_level);
-  d.task_sets.clear();
-  d.ts = nullptr;
+  d.clear_tasks();
   assign_tiers(cfg_.tc_min_front > 0 ? cfg_.tc_min_front : kTcDefaultMinFront);
   // The top of the tree for the backward sweep: the trailing levels of at
   // most kBackwardTopFronts fronts.
@@ -682,8 +718,7 @@ void Engine::analyze_host(int32_t n_bus, const int32_t* indptr, const int32_t* i
   so.par_nd_base_large = cfg_.par_nd_base_large;
   sp_ = analyze_symbolic(ja_.dim, ja_.row_ptr.data(), ja_.col_idx.data(), so);
   fp_ = build_factor_program(sp_);
-  d_->task_sets.clear();
-  d_->ts = nullptr;
+  d_->clear_tasks();
 }
 
 void Engine::analyze_matrix_host(int32_t n, int32_t nnz, const int32_t* row_ptr, const int32_t* col_idx) {
@@ -705,8 +740,7 @@ void Engine::analyze_matrix_host(int32_t n, int32_t nnz, const int32_t* row_ptr,
   so.par_nd_base_large = cfg_.par_nd_base_large;
   sp_ = analyze_symbolic(n, row_ptr, col_idx, so);
   fp_ = build_factor_program(sp_);
-  d_->task_sets.clear();
-  d_->ts = nullptr;
+  d_->clear_tasks();
 }
 
 void Engine::initialize_matrix(int32_t n, int32_t nnz, const int32_t* row_ptr, const int32_t* col_idx) {
@@ -726,8 +760,7 @@ void Engine::initialize_matrix(int32_t n, int32_t nnz, const int32_t* row_ptr, c
   so.par_nd_base_large = cfg_.par_nd_base_large;
   sp_ = analyze_symbolic(n, row_ptr, col_idx, so);
   fp_ = build_factor_program(sp_);
-  d_->task_sets.clear();
-  d_->ts = nullptr;
+  d_->clear_tasks();
   upload_plan();
   initialized_ = true;
   adjoint_ready_ = false;
@@ -740,8 +773,8 @@ void Engine::ensure_workspace(int32_t B) {
   const int Bp = (B + kWarp - 1) / kWarp * kWarp;
   d.B = B;
   d.Bp = Bp;
-  select_tasks();
   if (Bp > d.Bp_cap) {
+    prepare_tasks(Bp);
     const size_t n = ja_.n_bus, dim = ja_.dim;
     const size_t es = factor_is_double() ? sizeof(double) : sizeof(float);
     for (DBuf* b : {&d.v_re, &d.v_im, &d.va, &d.vm, &d.s_re, &d.s_im, &d.i_re, &d.i_im}) b->reserve(n * Bp * 8);
@@ -785,6 +818,7 @@ void Engine::ensure_workspace(int32_t B) {
     }
     adjoint_ready_ = false;
   }
+  select_tasks();
   if (Bp > d.h_cap) {
     if (d.h_norm) cudaFreeHost(d.h_norm);
     if (d.h_final) cudaFreeHost(d.h_final);
@@ -1100,19 +1134,24 @@ std::vector<int32_t> Engine::task_array(std::string name) const {
     cls = std::min(std::max(std::atoi(name.c_str() + colon + 1), 0), 3);
     name.resize(colon);
   }
-  const TaskSet& set = task_set(cls);
-  const TaskPlan& t = set.tasks;
-  if (name == "task_meta") return t.meta;
-  if (name == "task_words") return t.words;
-  if (name == "task_sweep_meta") return set.sweeps.meta;
-  if (name == "task_sweep_words") return set.sweeps.words;
-  if (name == "task_sweep_stages") {
+  if (name == "task_classes") {
+    std::vector<int32_t> c;
+    for (const auto& s : d_->task_sets) c.push_back(s.first);
+    return c;
+  }
+  if (name.compare(0, 10, "task_sweep") == 0) {
+    const SweepPlan sweeps = sweep_plan(cls);
+    if (name == "task_sweep_meta") return sweeps.meta;
+    if (name == "task_sweep_words") return sweeps.words;
     std::vector<int32_t> st;
-    for (const auto& s : set.sweeps.stages)
+    for (const auto& s : sweeps.stages)
       st.insert(st.end(), {s.begin, s.count, s.max_words, s.max_local, s.max_arena, s.max_rows, s.max_u, s.max_l,
                            s.warps});
     return st;
   }
+  const TaskPlan t = task_plan(cls);
+  if (name == "task_meta") return t.meta;
+  if (name == "task_words") return t.words;
   std::vector<int32_t> st;
   for (const auto& s : t.stages) st.insert(st.end(), {s.begin, s.count, s.max_words, s.max_arena, s.warps});
   return st;
@@ -1188,7 +1227,7 @@ int64_t Engine::launch_factor(const FactorArgs<T, T>& a, cudaStream_t s) {
     return n;
   }
   for (const auto& st : d.ts->tasks.stages) {
-    launch_factor_stage<T>(st, a, d.ts->task_meta.template as<int>(), d.ts->task_words.template as<int>(), d.task_lanes(), s);
+    launch_factor_stage<T>(st, a, d.ts->meta.template as<int>(), d.ts->words.template as<int>(), d.task_lanes(), s);
     debug_check(s, "factor tasks");
     ++n;
   }
@@ -1222,21 +1261,17 @@ void Engine::backward_all(cudaStream_t s) {
   stage_end(3, s);
 }
 
-// Small trees sweep level by level: factorize + solve + transpose solve with
-// 300 buses (about 250 fronts) x 20 takes 321 us by levels and 349 us by
-// tasks, 610 and 696 us x 1,500 in FP64; 500 buses (420 fronts) x 200 515 and
-// 448 us, 800 buses x 300 635 and 532 us.
-bool Engine::use_sweep_tasks() const { return !d_->ts->sweeps.stages.empty() && fp_.P >= 400; }
+bool Engine::use_sweep_tasks() const { return d_->sweeps && !d_->sweeps->plan.stages.empty(); }
 
 // One sweep over the subtree tasks (modes: launch_sweep_stage), a launch per stage.
 template <typename T>
 int64_t Engine::sweep_tasks(int mode, const SweepTaskArgs<T>& a, cudaStream_t s) {
   auto& d = *d_;
-  const SweepPlan& sp = d.ts->sweeps;
+  const SweepPlan& sp = d.sweeps->plan;
   const int n = (int)sp.stages.size();
   for (int i = 0; i < n; ++i) {
-    launch_sweep_stage<T>(mode, sp.stages[mode < 2 ? i : n - 1 - i], a, d.Bp / kWarp, d.ts->sweep_meta.template as<int>(),
-                          d.ts->sweep_words.template as<int>(), d.task_lanes(), s);
+    launch_sweep_stage<T>(mode, sp.stages[mode < 2 ? i : n - 1 - i], a, d.Bp / kWarp, d.sweeps->meta.template as<int>(),
+                          d.sweeps->words.template as<int>(), d.task_lanes(), s);
     debug_check(s, "sweep tasks");
   }
   return n;
@@ -1788,6 +1823,7 @@ void Engine::factorize_values_static_scratch(const void* d_values, int32_t value
                                 " bytes of front scratch, the static area holds " + std::to_string(scratch_bytes));
   d.B = B;
   d.Bp = Bp;
+  select_tasks();
   cudaStream_t s = stream ? stream : d.own;
   if (dbl) {
     if (values_is_double)

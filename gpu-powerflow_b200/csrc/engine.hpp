@@ -17,6 +17,7 @@
 #include "analysis.hpp"
 #include "device_plan.cuh"
 #include "kernels.hpp"
+#include "task_plan.hpp"
 
 namespace cupf_b200 {
 
@@ -126,7 +127,8 @@ class Engine {
   // the factorization's subtree tasks (task_plan.hpp): "task_meta", "task_words",
   // "task_stages" (per stage: first task, tasks, largest program and arena, warps of
   // a team); the sweeps': "task_sweep_meta", "task_sweep_words",
-  // "task_sweep_stages"; ":c" after a name picks the batch class (default 3)
+  // "task_sweep_stages"; ":c" after a name picks the batch class (default 3);
+  // "task_classes": the classes whose factorization plans are on the device
   std::vector<int32_t> task_array(std::string name) const;
   int32_t tc_threshold() const { return tc_min_; }
   // the same for the backward sweep's launches, tree top first
@@ -154,6 +156,7 @@ class Engine {
  private:
   struct Impl;
   struct TaskSet;
+  struct SweepSet;
   std::unique_ptr<Impl> d_;
   EngineConfig cfg_;
   JacobianAnalysis ja_;
@@ -174,7 +177,9 @@ class Engine {
 
   void ensure_workspace(int32_t B);
   void upload_plan();
-  TaskSet& task_set(int cls) const;
+  TaskPlan task_plan(int cls) const;
+  SweepPlan sweep_plan(int cls) const;
+  void prepare_tasks(int32_t B);
   void select_tasks();
   template <typename Buf>
   void pad_lists(std::vector<LevelLaunch>& levels, const std::vector<int32_t>& order, Buf& src, Buf& dst) const;

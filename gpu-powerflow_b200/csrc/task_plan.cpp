@@ -557,7 +557,7 @@ std::vector<TaskStageSpec> factor_task_specs(int cls, int elem_bytes) {
 // takes wider groups of scenarios per team and joined subtrees.
 std::vector<TaskStageSpec> sweep_task_specs(int cls) {
   // cut, merge, arena, words, factor elements, warps, lanes, pack
-  if (cls == 3)
+  if (sweep_class(cls) == 3)
     return {{400, 1200, 60, 4000, 80, 1, 16, 1}, {1500, 1500, 160, 4000, 150, 1, 16, 1},
             {0, 0, 2400, 11000, 640, 2, 8, 1}};
   return {{500, 0, 160, 4000, 150, 1, 8, 1}, {2500, 0, 2400, 11000, 640, 2, 8, 1}, {0, 0, 2400, 11000, 640, 2, 8, 1}};

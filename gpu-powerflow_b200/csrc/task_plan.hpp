@@ -59,6 +59,7 @@ struct TaskStageSpec {
 // Classes of batches with stages of their own: 0 a single system; by the
 // fronts x systems of a batch, 1 little, 2 medium, 3 much work.
 int task_class(int fronts, int batch);
+constexpr int sweep_class(int cls) { return cls == 3 ? 3 : 0; }  // classes with the same sweep stages
 // The stages of a class, for 4- or 8-byte factors.
 std::vector<TaskStageSpec> factor_task_specs(int cls, int elem_bytes);
 std::vector<TaskStageSpec> sweep_task_specs(int cls);

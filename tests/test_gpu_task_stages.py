@@ -69,6 +69,33 @@ def test_first_solves_on_a_side_stream_wait_for_their_plans():
         assert torch.equal(got, want)
 
 
+def test_smaller_batches_plan_and_allocate_nothing():
+    """The plans of every class a workspace serves come with it; a tree below
+    the thresholds gets none."""
+    import torch
+
+    def solve(s, g, batch):
+        S = torch.tensor(g.scenarios(batch, seed=batch), device="cuda")
+        s.solve_batch_device(S, torch.tensor(g.flat_start(batch), device="cuda"),
+                             config=cupf.NRConfig(tolerance=1e-8, max_iter=10))
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    small = _newton(_grid(118), "Mixed", autotune=False)
+    solve(small, _grid(118), 300)
+    assert small.plan_array("task_classes").size == 0
+    g = _grid(4000)
+    s = _newton(g, "Mixed", autotune=False)
+    solve(s, g, 288)
+    assert s.plan_array("task_classes").tolist() == [0, 1, 2, 3]
+    for batch in (1, 20, 160):  # inputs of these sizes first, so that torch's pool holds them
+        torch.tensor(g.scenarios(batch, seed=batch), device="cuda"), torch.tensor(g.flat_start(batch), device="cuda")
+    free = solve(s, g, 288)
+    for batch in (160, 20, 1):  # the other classes
+        assert solve(s, g, batch) == free
+    assert s.plan_array("task_classes").tolist() == [0, 1, 2, 3]
+
+
 def _linear(g, precision, **config):
     h = cupf.NewtonSolver(cupf.NewtonOptions(backend=cupf.BackendKind.CUDA))
     h.analyze_host(g.indptr, g.indices, g.n_bus, g.pv, g.pq)
