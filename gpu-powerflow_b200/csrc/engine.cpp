@@ -766,6 +766,20 @@ void Engine::initialize_matrix(int32_t n, int32_t nnz, const int32_t* row_ptr, c
   adjoint_ready_ = false;
 }
 
+// The global front scratch (elements x 32) that one of these launches can need,
+// whatever tier and placement it is given.
+size_t Engine::scratch_capacity(const std::vector<LevelLaunch>& levels, int groups) const {
+  const size_t es = factor_is_double() ? sizeof(double) : sizeof(float);
+  size_t scratch = 0;
+  for (const auto& lv : levels) {
+    LevelLaunch widest = lv;  // the tier with the largest scratch this launch may be given
+    if (tf32_factors() && lv.max_fsz >= std::min(tc_min_ > 0 ? tc_min_ : kTcSmallestMinFront, kTcSmallestMinFront))
+      widest.tier = 2;
+    scratch = std::max({scratch, level_scratch_capacity(lv, es, groups), level_scratch_capacity(widest, es, groups)});
+  }
+  return scratch;
+}
+
 void Engine::ensure_workspace(int32_t B) {
   if (!initialized_) throw std::runtime_error("NewtonSolver::solve_batch(): initialize() must be called first");
   if (B <= 0) throw std::invalid_argument("NewtonSolver::solve_batch(): batch_size must be positive");
@@ -795,14 +809,10 @@ void Engine::ensure_workspace(int32_t B) {
     d.X.reserve(dim * Bp * es);
     // dense fronts of levels too large for shared memory (and every wide-tier
     // front) live in global scratch; one launch at a time uses it
-    size_t scratch = 0;
-    for (const auto& lv : d.levels) {
-      LevelLaunch widest = lv;  // the tier with the largest scratch this launch may be given
-      if (tf32_factors() && lv.max_fsz >= std::min(tc_min_ > 0 ? tc_min_ : kTcSmallestMinFront, kTcSmallestMinFront))
-        widest.tier = 2;
-      scratch = std::max({scratch, level_scratch_capacity(lv, es, Bp / kWarp),
-                          level_scratch_capacity(widest, es, Bp / kWarp)});
-    }
+    // (the launches of the fronts that tasks leave are cut anew: with fewer
+    // fronts one launch may join more of them than a level's launches do)
+    size_t scratch = scratch_capacity(d.levels, Bp / kWarp);
+    for (const auto& ts : d.task_sets) scratch = std::max(scratch, scratch_capacity(ts.second->rest, Bp / kWarp));
     d.front_scratch_elems = scratch;
     if (scratch) d.front_scratch.reserve(scratch * kWarp * es);
     // The allocation-free entry point's static area: the runtime loads the

@@ -180,6 +180,7 @@ class Engine {
   TaskPlan task_plan(int cls) const;
   SweepPlan sweep_plan(int cls) const;
   void prepare_tasks(int32_t B);
+  size_t scratch_capacity(const std::vector<LevelLaunch>& levels, int groups) const;
   void select_tasks();
   template <typename Buf>
   void pad_lists(std::vector<LevelLaunch>& levels, const std::vector<int32_t>& order, Buf& src, Buf& dst) const;

@@ -138,3 +138,37 @@ def test_batch_of_one_sweeps_equal_the_lane_kernels(buses, precision):
         ls.factorize(A)
         out.append((ls.solve(b), ls.solve_transpose(b)))
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
+def test_launches_beside_tasks_fit_the_front_scratch():
+    """Fronts that an option keeps off the tasks run in launches of their own,
+    cut anew.  Dense blocks of 18, 20 and 28 rows in panels of 4: the leaf
+    level's launches are 70 fronts of 18 and 20 rows and 64 of 28; without the
+    blocks of 18, which the tasks take, the 40 and the 64 are one launch of 104
+    at 28 rows, which needs more scratch than either."""
+    import scipy.sparse as sp
+    import torch
+
+    rng = np.random.default_rng(3)
+    sizes = [18] * 30 + [20] * 40 + [28] * 64
+    A = sp.block_diag([sp.coo_array(np.ones((n, n))) for n in sizes]).tocsr()
+    A.sort_indices()
+    n = A.shape[0]
+    ls = cupf.LinearSolver(cupf.SolverConfig(precision=int(cupf.CustomPrecision.FP64), serial_nd=True,
+                                             max_panel_width=4, wide_min_front=20, autotune=False))
+    ls.set_data(A.indptr.astype(np.int32), A.indices.astype(np.int32))
+    ls.analyze()
+    fsz = ls.plan_array("fp_fsz")
+    assert fsz.size >= 300 and fsz.max() == 28
+    B = 2
+    vals = rng.standard_normal((B, A.nnz))
+    rows = np.repeat(np.arange(n), np.diff(A.indptr))
+    vals[:, rows == A.indices] += 24.0
+    b = rng.standard_normal((B, n))
+    ls.setup(B)
+    ls.factorize(torch.tensor(vals, device="cuda"))
+    x = ls.solve(torch.tensor(b, device="cuda")).cpu().numpy()
+    for k in range(B):
+        M = sp.csr_matrix((vals[k], A.indices, A.indptr), shape=(n, n))
+        # diagonally dominant: growth below 2, n = 28 rows to a block
+        assert np.linalg.norm(M @ x[k] - b[k]) <= 1e-13 * np.linalg.norm(b[k])
