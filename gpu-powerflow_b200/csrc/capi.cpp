@@ -121,7 +121,7 @@ bool copy_plan_array(const Engine& e, const char* name, int32_t* out, int64_t ca
   if (n == "factor_level_warps" || n == "backward_launch_warps" || n == "factor_level_tiers" ||
       n == "tc_threshold" || n == "factor_level_placement" ||  // the autotuner's choices, each launch's kernel
       n.compare(0, 9, "task_meta") == 0 || n.compare(0, 10, "task_words") == 0 ||
-      n.compare(0, 11, "task_stages") == 0 || n == "task_classes" || n.compare(0, 11, "task_sweep_") == 0) {
+      n.compare(0, 11, "task_stages") == 0 || n == "task_classes" || n == "task_class" || n.compare(0, 11, "task_sweep_") == 0) {
     const std::vector<int32_t> w = n.compare(0, 5, "task_") == 0  ? e.task_array(n)
                                    : n == "factor_level_warps"    ? e.factor_level_warps()
                                    : n == "factor_level_tiers"     ? e.factor_level_tiers()

@@ -463,14 +463,14 @@ SweepPlan Engine::sweep_plan(int cls) const {
 }
 
 // Builds and uploads the plans of every class that a batch of up to B systems
-// can have, so that a smaller batch on this workspace allocates and plans
+// (a multiple of 32) can have, so that a smaller batch on this workspace allocates and plans
 // nothing; trees below the thresholds, which use neither, get none.  All four
 // classes take about as long as the symbolic analysis (2,000 buses: 15 ms).
 void Engine::prepare_tasks(int32_t B) {
   auto& d = *d_;
   std::vector<int> classes{task_class(fp_.P, 1)};
   if (B > 1)  // (the classes of larger batches follow one another)
-    for (int c = task_class(fp_.P, 2); c <= task_class(fp_.P, B); ++c) classes.push_back(c);
+    for (int c = task_class(fp_.P, kWarp); c <= task_class(fp_.P, B); ++c) classes.push_back(c);
   for (int cls : classes) {
     if (fp_.P >= kTaskFronts && !d.task_sets.count(cls)) {
       auto ts = std::make_unique<TaskSet>();
@@ -512,7 +512,8 @@ void Engine::prepare_tasks(int32_t B) {
 // Makes the current batch's plans the ones in use.
 void Engine::select_tasks() {
   auto& d = *d_;
-  const int cls = task_class(fp_.P, d.B);
+  // by the padded batch, which the captured solve and the tuned shapes go by too
+  const int cls = task_class(fp_.P, d.B == 1 ? 1 : d.Bp);
   const auto ts = d.task_sets.find(cls);
   const auto ss = d.sweep_sets.find(sweep_class(cls));
   d.ts = ts == d.task_sets.end() ? nullptr : ts->second.get();
@@ -1144,6 +1145,10 @@ std::vector<int32_t> Engine::task_array(std::string name) const {
     cls = std::min(std::max(std::atoi(name.c_str() + colon + 1), 0), 3);
     name.resize(colon);
   }
+  if (name == "task_class")
+    for (const auto& s : d_->task_sets)
+      if (s.second.get() == d_->ts && use_tasks()) return {s.first};
+  if (name == "task_class") return {-1};
   if (name == "task_classes") {
     std::vector<int32_t> c;
     for (const auto& s : d_->task_sets) c.push_back(s.first);

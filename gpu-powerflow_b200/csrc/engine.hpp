@@ -128,7 +128,8 @@ class Engine {
   // "task_stages" (per stage: first task, tasks, largest program and arena, warps of
   // a team); the sweeps': "task_sweep_meta", "task_sweep_words",
   // "task_sweep_stages"; ":c" after a name picks the batch class (default 3);
-  // "task_classes": the classes whose factorization plans are on the device
+  // "task_classes": the classes whose factorization plans are on the device;
+  // "task_class": the class whose tasks factor the current batch, -1 when none do
   std::vector<int32_t> task_array(std::string name) const;
   int32_t tc_threshold() const { return tc_min_; }
   // the same for the backward sweep's launches, tree top first

@@ -96,6 +96,24 @@ def test_smaller_batches_plan_and_allocate_nothing():
     assert s.plan_array("task_classes").tolist() == [0, 1, 2, 3]
 
 
+@pytest.mark.parametrize("first,second", [(470, 479), (479, 470)])
+def test_one_padded_batch_has_one_class(first, second):
+    """500 buses are 420 fronts: 420 x 476 systems is where class 2 begins, and
+    470 and 479 systems have the same padded batch, whose captured solve and
+    tuned shapes they share."""
+    import torch
+
+    g = _grid(500)
+    s = _newton(g, "Mixed", graph=True, autotune=False)
+    cls = []
+    for batch in (first, second):
+        S = torch.tensor(g.scenarios(batch, seed=batch), device="cuda")
+        s.solve_batch_device(S, torch.tensor(g.flat_start(batch), device="cuda"),
+                             config=cupf.NRConfig(tolerance=1e-8, max_iter=10))
+        cls += s.plan_array("task_class").tolist()
+    assert cls == [2, 2]
+
+
 def _linear(g, precision, **config):
     h = cupf.NewtonSolver(cupf.NewtonOptions(backend=cupf.BackendKind.CUDA))
     h.analyze_host(g.indptr, g.indices, g.n_bus, g.pv, g.pq)
