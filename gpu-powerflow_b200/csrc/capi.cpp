@@ -118,16 +118,20 @@ bool copy_plan_array(const Engine& e, const char* name, int32_t* out, int64_t ca
   CUPF_ARR("diag12", ja.diag12)
   CUPF_ARR("diag22", ja.diag22)
 #undef CUPF_ARR
-  if (n == "factor_level_warps" || n == "backward_launch_warps" || n == "factor_level_tiers" ||
-      n == "tc_threshold" || n == "factor_level_placement" ||  // the autotuner's choices, each launch's kernel
-      n.compare(0, 9, "task_meta") == 0 || n.compare(0, 10, "task_words") == 0 ||
-      n.compare(0, 11, "task_stages") == 0 || n == "task_classes" || n == "task_class" || n.compare(0, 11, "task_sweep_") == 0) {
-    const std::vector<int32_t> w = n.compare(0, 5, "task_") == 0  ? e.task_array(n)
-                                   : n == "factor_level_warps"    ? e.factor_level_warps()
-                                   : n == "factor_level_tiers"     ? e.factor_level_tiers()
-                                   : n == "factor_level_placement" ? e.factor_level_placements()
-                                   : n == "tc_threshold"           ? std::vector<int32_t>{e.tc_threshold()}
-                                                                   : e.backward_launch_warps();
+  // the launch plan: the autotuner's choices, each launch's kernel, the tasks
+  std::vector<int32_t> w;
+  bool known = true;
+  if (n == "factor_level_warps") w = e.factor_level_warps();
+  else if (n == "factor_level_tiers") w = e.factor_level_tiers();
+  else if (n == "factor_level_placement") w = e.factor_level_placements();
+  else if (n == "factor_rest_warps") w = e.factor_level_warps(true);
+  else if (n == "factor_rest_tiers") w = e.factor_level_tiers(true);
+  else if (n == "factor_rest_placement") w = e.factor_level_placements(true);
+  else if (n == "factor_tuned_launches") w = e.factor_tuned_launches();
+  else if (n == "backward_launch_warps") w = e.backward_launch_warps();
+  else if (n == "tc_threshold") w = {e.tc_threshold()};
+  else known = e.task_array(n, &w);
+  if (known) {
     if (len) *len = (int64_t)w.size();
     if (out) {
       if (cap < (int64_t)w.size()) return false;

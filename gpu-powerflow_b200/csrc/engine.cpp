@@ -186,7 +186,8 @@ struct Engine::Impl {
   LoopCtl* h_ctl = nullptr;    // pinned
   // batch size and precision the factor and backward launches were tuned for
   int tuned_Bp = -1, tuned_bw_Bp = -1;
-  bool tuned_double = false, tuned_bw_double = false, tuned_single = false;
+  bool tuned_double = false, tuned_bw_double = false, tuned_single = false, tuned_tasks = false;
+  std::vector<int32_t> tuned_launches;  // timed at the last tuning: the rest launches, the level launches
   bool graph_single = false;  // the graph's factor launches use the single-system schedule
   void invalidate_graph() {
     if (exec) cudaGraphExecDestroy(exec);
@@ -287,9 +288,15 @@ void Engine::assign_tiers(int tc_min) {
     }
 }
 
-std::vector<int32_t> Engine::factor_level_tiers() const {
+// The level launches of the whole tree, or of the fronts the tasks of the current batch leave.
+const std::vector<LevelLaunch>& Engine::reported_levels(bool rest) const {
+  static const std::vector<LevelLaunch> none;
+  return !rest ? d_->levels : d_->ts && use_tasks() ? d_->ts->rest : none;
+}
+
+std::vector<int32_t> Engine::factor_level_tiers(bool rest) const {
   std::vector<int32_t> t;
-  for (const auto& lv : d_->levels) t.push_back(lv.tier);
+  for (const auto& lv : reported_levels(rest)) t.push_back(lv.tier);
   return t;
 }
 
@@ -1012,18 +1019,24 @@ bool choose_block_shapes(size_t n, const std::vector<int>& cand, Set set, Launch
 // The autotuner of the factor launches: each block factors one front for 32
 // scenarios and its warps split the staging, the assembly and the non-pivot
 // rows, so every element sees the same operations in the same order whatever
-// the split.  Tunes once per batch size and precision, on the values J.
+// the split.  Tunes the launches that factor this batch, once per batch size
+// and precision, on the values J; all_levels: the level launches of the whole
+// tree too, which the allocation-free factorization runs.
 template <typename T>
-void Engine::autotune_factor(cudaStream_t s, const void* J) {
+void Engine::autotune_factor(cudaStream_t s, const void* J, bool all_levels) {
   auto& d = *d_;
   const bool dbl = std::is_same<T, double>::value;
-  if (d.tuned_Bp == d.Bp && d.tuned_double == dbl && d.tuned_single == single_system()) return;
+  if (d.tuned_Bp == d.Bp && d.tuned_double == dbl && d.tuned_single == single_system() &&
+      d.tuned_tasks == use_tasks())
+    return;
+  d.tuned_launches = {0, 0};
   if (single_system()) {
     // batch 1: the single-system kernel has no launch shapes to choose (the
     // tensor-core threshold of TF32 factors stays at its default)
     d.tuned_Bp = d.Bp;
     d.tuned_double = dbl;
     d.tuned_single = true;
+    d.tuned_tasks = use_tasks();
     d.invalidate_graph();
     return;
   }
@@ -1076,23 +1089,32 @@ void Engine::autotune_factor(cudaStream_t s, const void* J) {
   for (int p : {1, 2})
     for (int w : {1, 2, 4, 8}) cand.push_back(w + 256 * p);
   for (int w : {8, 16, 32}) cand.push_back(w + 256 * 3);
+  const auto tune = [&](std::vector<LevelLaunch>& levels, const FactorArgs<T, T>& la) {
+    choose_block_shapes(
+        levels.size(), cand,
+        [&](size_t i, int code) {
+          LevelLaunch& lv = levels[i];
+          int w = code & 0xff, p = code >> 8;
+          if (p == 3 && !(lv.tier == 1 || wide_option(lv))) w = p = 0;
+          lv.warps = w;
+          lv.placement = lv.tier == 0 ? p : 0;
+        },
+        [&](size_t i) { launch_factor_level<T, T>(levels[i], la, s); }, s, "factor");
+  };
   const bool tasks = use_tasks();
-  std::vector<LevelLaunch>& levels = tasks ? d.ts->rest : d.levels;
-  const FactorArgs<T, T> la = tasks ? rest_args<T>(a) : a;
-  if (tasks) launch_factor<T>(a, s);  // (the level launches read the tasks' contribution blocks)
-  choose_block_shapes(
-      levels.size(), cand,
-      [&](size_t i, int code) {
-        LevelLaunch& lv = levels[i];
-        int w = code & 0xff, p = code >> 8;
-        if (p == 3 && !(lv.tier == 1 || wide_option(lv))) w = p = 0;
-        lv.warps = w;
-        lv.placement = lv.tier == 0 ? p : 0;
-      },
-      [&](size_t i) { launch_factor_level<T, T>(levels[i], la, s); }, s, "factor");
+  if (tasks) {
+    launch_factor<T>(a, s);  // (the rest launches read the tasks' contribution blocks)
+    tune(d.ts->rest, rest_args<T>(a));
+    d.tuned_launches[0] = (int32_t)d.ts->rest.size();
+  }
+  if (!tasks || all_levels) {
+    tune(d.levels, a);
+    d.tuned_launches[1] = (int32_t)d.levels.size();
+  }
   d.tuned_Bp = d.Bp;
   d.tuned_double = dbl;
   d.tuned_single = false;
+  d.tuned_tasks = tasks;
   d.invalidate_graph();  // a captured solve holds the old launch shapes
 }
 
@@ -1138,50 +1160,60 @@ SweepArgs<T> Engine::sweep_args() const {
   return a;
 }
 
-std::vector<int32_t> Engine::task_array(std::string name) const {
+bool Engine::task_array(std::string name, std::vector<int32_t>* out) const {
+  out->clear();
+  if (name == "task_class") {
+    out->push_back(-1);
+    for (const auto& s : d_->task_sets)
+      if (s.second.get() == d_->ts && use_tasks()) (*out)[0] = s.first;
+    return true;
+  }
+  if (name == "task_classes") {
+    for (const auto& s : d_->task_sets) out->push_back(s.first);
+    return true;
+  }
   int cls = 3;  // "name:class"
   const size_t colon = name.find(':');
   if (colon != std::string::npos) {
-    cls = std::min(std::max(std::atoi(name.c_str() + colon + 1), 0), 3);
+    const std::string c = name.substr(colon + 1);
+    if (c.size() != 1 || c[0] < '0' || c[0] > '3') return false;
+    cls = c[0] - '0';
     name.resize(colon);
   }
-  if (name == "task_class")
-    for (const auto& s : d_->task_sets)
-      if (s.second.get() == d_->ts && use_tasks()) return {s.first};
-  if (name == "task_class") return {-1};
-  if (name == "task_classes") {
-    std::vector<int32_t> c;
-    for (const auto& s : d_->task_sets) c.push_back(s.first);
-    return c;
+  if (name == "task_meta" || name == "task_words" || name == "task_stages") {
+    TaskPlan t = task_plan(cls);
+    if (name == "task_meta") *out = std::move(t.meta);
+    else if (name == "task_words") *out = std::move(t.words);
+    else
+      for (const auto& s : t.stages)
+        out->insert(out->end(), {s.begin, s.count, s.max_words, s.max_arena, s.warps});
+    return true;
   }
-  if (name.compare(0, 10, "task_sweep") == 0) {
-    const SweepPlan sweeps = sweep_plan(cls);
-    if (name == "task_sweep_meta") return sweeps.meta;
-    if (name == "task_sweep_words") return sweeps.words;
-    std::vector<int32_t> st;
-    for (const auto& s : sweeps.stages)
-      st.insert(st.end(), {s.begin, s.count, s.max_words, s.max_local, s.max_arena, s.max_rows, s.max_u, s.max_l,
-                           s.warps});
-    return st;
+  if (name == "task_sweep_meta" || name == "task_sweep_words" || name == "task_sweep_stages") {
+    SweepPlan t = sweep_plan(cls);
+    if (name == "task_sweep_meta") *out = std::move(t.meta);
+    else if (name == "task_sweep_words") *out = std::move(t.words);
+    else
+      for (const auto& s : t.stages)
+        out->insert(out->end(), {s.begin, s.count, s.max_words, s.max_local, s.max_arena, s.max_rows, s.max_u,
+                                 s.max_l, s.warps});
+    return true;
   }
-  const TaskPlan t = task_plan(cls);
-  if (name == "task_meta") return t.meta;
-  if (name == "task_words") return t.words;
-  std::vector<int32_t> st;
-  for (const auto& s : t.stages) st.insert(st.end(), {s.begin, s.count, s.max_words, s.max_arena, s.warps});
-  return st;
+  return false;
 }
 
-std::vector<int32_t> Engine::factor_level_warps() const {
+std::vector<int32_t> Engine::factor_tuned_launches() const { return d_->tuned_launches; }
+
+std::vector<int32_t> Engine::factor_level_warps(bool rest) const {
   std::vector<int32_t> w;
-  for (const auto& lv : d_->levels) w.push_back(lv.warps);
+  for (const auto& lv : reported_levels(rest)) w.push_back(lv.warps);
   return w;
 }
 
-std::vector<int32_t> Engine::factor_level_placements() const {
+std::vector<int32_t> Engine::factor_level_placements(bool rest) const {
   std::vector<int32_t> p;
   const size_t es = factor_is_double() ? sizeof(double) : sizeof(float);
-  for (const auto& lv : d_->levels)
+  for (const auto& lv : reported_levels(rest))
     p.push_back(lv.tier > 0 ? 2 : runs_wide(lv, es) ? 3 : (front_in_shared_memory(lv, es) ? 1 : 2));
   return p;
 }
@@ -1420,11 +1452,12 @@ SolveStats Engine::run_loop(double tol, int32_t max_iter, int32_t prepare_adjoin
   adjoint_ready_ = false;
   if (cfg_.autotune && max_iter > 0 &&
       (d.tuned_Bp != d.Bp || d.tuned_double != std::is_same<T, double>::value || d.tuned_bw_Bp != d.Bp ||
-       d.tuned_bw_double != std::is_same<T, double>::value || d.tuned_single != single_system())) {
+       d.tuned_bw_double != std::is_same<T, double>::value || d.tuned_single != single_system() ||
+       d.tuned_tasks != use_tasks())) {
     // tune on the Jacobian of the starting state (the loop recomputes it)
     launch_ibus_mismatch(d.g, st, s);
     launch_jacobian<T>(d.g, st, d.J.as<T>(), s);
-    autotune_factor<T>(s, d.J.p);
+    autotune_factor<T>(s, d.J.p, false);
     autotune_backward<T>(s);  // on the factors the factor tuning left
   }
   CUPF_CUDA(cudaMemsetAsync(d.norm.p, 0, d.Bp * sizeof(unsigned long long), s));
@@ -1766,8 +1799,8 @@ void Engine::factorize_values(const void* d_values, int32_t values_is_double, in
   CUPF_CUDA(cudaMemsetAsync(d.F.p, 0, (size_t)ja_.dim * d.Bp * 8, s));
   CUPF_CUDA(cudaMemsetAsync(d.Fp.p, 0, (size_t)ja_.dim * d.Bp * (dbl ? 8 : 4), s));
   if (cfg_.autotune) {
-    if (dbl) autotune_factor<double>(s, d.J.p);
-    else autotune_factor<float>(s, d.J.p);
+    if (dbl) autotune_factor<double>(s, d.J.p, true);
+    else autotune_factor<float>(s, d.J.p, true);
   }
   CUPF_CUDA(cudaMemsetAsync(d.sing.p, 0, d.Bp * sizeof(int), s));
   if (dbl) factor_all<double>(s, 1, d.J.p);

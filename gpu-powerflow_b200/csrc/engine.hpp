@@ -117,20 +117,26 @@ class Engine {
 
   const JacobianAnalysis& jacobian() const { return ja_; }
   const SymbolicPlan& symbolic() const { return sp_; }
-  // warps per block of each factor level launch (0: the built-in rule)
-  std::vector<int32_t> factor_level_warps() const;
-  // factor kernel tier of each launch (0 register rows, 1 any-size, 2 tensor
-  // cores) and the tensor-core threshold in use (0 when not TF32)
-  std::vector<int32_t> factor_level_tiers() const;
-  // where each factor launch keeps its dense fronts: 1 shared memory, 2 the global scratch
-  std::vector<int32_t> factor_level_placements() const;
+  // The level launches of the whole tree (small trees, the allocation-free
+  // factorization), or with rest those of the fronts that the tasks of the
+  // current batch leave (empty when no tasks run).  Warps per block of each
+  // (0: the built-in rule) ...
+  std::vector<int32_t> factor_level_warps(bool rest = false) const;
+  // ... its kernel tier (0 register rows, 1 any-size, 2 tensor
+  // cores; the tensor-core threshold in use is 0 when not TF32) ...
+  std::vector<int32_t> factor_level_tiers(bool rest = false) const;
+  // ... and where it keeps its dense fronts: 1 shared memory, 2 the global scratch
+  std::vector<int32_t> factor_level_placements(bool rest = false) const;
+  // launches the last tuning of the factorization timed: rest launches, level launches
+  std::vector<int32_t> factor_tuned_launches() const;
   // the factorization's subtree tasks (task_plan.hpp): "task_meta", "task_words",
   // "task_stages" (per stage: first task, tasks, largest program and arena, warps of
   // a team); the sweeps': "task_sweep_meta", "task_sweep_words",
   // "task_sweep_stages"; ":c" after a name picks the batch class (default 3);
   // "task_classes": the classes whose factorization plans are on the device;
   // "task_class": the class whose tasks factor the current batch, -1 when none do
-  std::vector<int32_t> task_array(std::string name) const;
+  // (false: no such name)
+  bool task_array(std::string name, std::vector<int32_t>* out) const;
   int32_t tc_threshold() const { return tc_min_; }
   // the same for the backward sweep's launches, tree top first
   std::vector<int32_t> backward_launch_warps() const;
@@ -223,7 +229,8 @@ class Engine {
   // times every factor level with each candidate block shape on the values J
   // and keeps the fastest per level (once per batch size and precision)
   template <typename T>
-  void autotune_factor(cudaStream_t s, const void* J);
+  void autotune_factor(cudaStream_t s, const void* J, bool all_levels);
+  const std::vector<LevelLaunch>& reported_levels(bool rest) const;
   template <typename T>
   void autotune_backward(cudaStream_t s);
   template <typename T>

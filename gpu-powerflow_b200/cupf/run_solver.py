@@ -115,11 +115,13 @@ def main(argv=None) -> int:
         if xth is not None:
             rest.append(float(np.linalg.norm(A.T @ xth[b] - rhs) / max(np.linalg.norm(rhs), 1e-300)))
     fsz = ls.plan_array("fp_fsz")
+    tasks = bool(ls.plan_array("task_class")[0] >= 0)  # the levels are then those of the fronts the tasks leave
     extra = {"solve_transpose_ms": round(statistics.median(tt), 4),
              "max_relative_residual_transpose": max(rest)} if args.transpose else {}
     print(json.dumps({
         "n": int(n), "nnz": int(ci.size), "batch": B, "precision": args.precision, "fronts": int(fsz.size),
-        "max_front": int(fsz.max()), "factor_level_tiers": ls.plan_array("factor_level_tiers").tolist(),
+        "max_front": int(fsz.max()), "factor_tasks": tasks,
+        "factor_level_tiers": ls.plan_array("factor_rest_tiers" if tasks else "factor_level_tiers").tolist(),
         "tc_threshold": int(ls.plan_array("tc_threshold")[0]),
         "factorize_ms": round(statistics.median(tf), 4), "solve_ms": round(statistics.median(ts), 4),
         "max_relative_residual": max(res), **extra, "singular": int(ls.singular_flags().sum())}))

@@ -158,14 +158,22 @@ const char* cls_last_error(cls_handle h);
  * "front_off", "a_pos_csr", "graph_xadj", "graph_adjncy", "sym_col_ptr",
  * "sym_row_idx"), or of the engine's launch plan: "factor_level_warps" and
  * "backward_launch_warps" (the autotuner's block shapes, 0 = built-in rule),
- * "factor_level_tiers" (per factor launch: 0 register-row kernel, 1 any-size
+ * "factor_level_tiers" (per factor level launch: 0 register-row kernel, 1 any-size
  * tier, 2 any-size tier with the tensor-core trailing update),
- * "factor_level_placement" (per factor launch: 1 dense fronts in shared
+ * "factor_level_placement" (per factor level launch: 1 dense fronts in shared
  * memory, 2 in the global scratch, 3 a register-tier launch of large fronts
  * run by the any-size tier instead; the autotuner chooses it with the block
  * shape, and a launch of the any-size tier may take 16 or 32 warps) and
  * "tc_threshold" (one value: the front size from which TF32 factors use the
- * tensor cores, 0 for other precisions).  With out == NULL only *len is set. */
+ * tensor cores, 0 for other precisions).  The factor_level arrays describe the
+ * launches of the whole tree, which factor small trees and run in
+ * cls_factorize_static_scratch.  Trees of 300 fronts and more otherwise factor
+ * as subtree tasks ("task_class": the class of the current batch's tasks, -1
+ * when none run; "task_classes": the classes planned on the device), and
+ * "factor_rest_warps", "factor_rest_tiers" and "factor_rest_placement" are the
+ * same for the launches of the fronts that the tasks leave;
+ * "factor_tuned_launches" counts the launches that the autotuner timed last (rest,
+ * level).  With out == NULL only *len is set. */
 cls_status cls_plan_array(cls_handle h, const char* name, int32_t* out, int64_t capacity, int64_t* len);
 /* Writes the per-front structure of the analysed plan to a CSV file:
  * q,p,fsz,nc,uc,level,parent,asm_len,extend_elems, the columns of the

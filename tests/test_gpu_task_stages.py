@@ -96,6 +96,62 @@ def test_smaller_batches_plan_and_allocate_nothing():
     assert s.plan_array("task_classes").tolist() == [0, 1, 2, 3]
 
 
+@pytest.mark.parametrize("policy", ["FP64", "Mixed"])
+@pytest.mark.parametrize("buses,wide", [(200, 0), (2000, 12)])
+def test_autotuner_times_the_launches_that_factor(buses, wide, policy):
+    """Plans that do run level launches: a tree below the tasks' threshold, and
+    the fronts of 12 rows and more (with their ancestors) beside the tasks.
+    The tuner times every one of them, and the solves keep their bits."""
+    import torch
+
+    g = _grid(buses)
+    base = _newton(g, policy, autotune=False, wide_min_front=wide)
+    tuned = _newton(g, policy, autotune=True, wide_min_front=wide)
+    for batch in (96, 256, 96):
+        S = torch.tensor(g.scenarios(batch, seed=9), device="cuda")
+        V0 = torch.tensor(g.flat_start(batch), device="cuda")
+        cfg = cupf.NRConfig(tolerance=1e-8, max_iter=12)
+        assert torch.equal(base.solve_batch_device(S, V0, config=cfg)[0], tuned.solve_batch_device(S, V0, config=cfg)[0])
+        n = tuned.plan_array("factor_rest_warps" if wide else "factor_level_warps").size
+        assert n > 0 and tuned.plan_array("factor_tuned_launches").tolist() == ([n, 0] if wide else [0, n])
+        assert (tuned.plan_array("task_class")[0] >= 0) == bool(wide)
+        if wide:
+            assert (tuned.plan_array("factor_rest_tiers") == 1).any()
+
+
+@pytest.mark.parametrize("schedule_first", [True, False])
+def test_batches_of_one_and_of_many_tune_their_own_launches(schedule_first):
+    """A batch of one on the lane kernels (batch1_schedule = 1) runs the level
+    launches, a batch of 20 the tasks and their rest: neither passes for the
+    other's tuning, though their padded batch is the same."""
+    import torch
+
+    g = _grid(500)
+    s = _newton(g, "Mixed", autotune=True, batch1_schedule=1, wide_min_front=12)
+    for batch in ((1, 20) if schedule_first else (20, 1)):
+        S = torch.tensor(g.scenarios(batch, seed=9), device="cuda")
+        s.solve_batch_device(S, torch.tensor(g.flat_start(batch), device="cuda"),
+                             config=cupf.NRConfig(tolerance=1e-8, max_iter=12))
+        rest, level = s.plan_array("factor_tuned_launches").tolist()
+        assert (level > 0 and rest == 0) if batch == 1 else (rest > 0 and level == 0)
+
+
+def test_static_scratch_factorization_keeps_its_tuning():
+    """cls_factorize_static_scratch runs the level launches, so cls_factorize
+    tunes those beside what it runs itself."""
+    import torch
+
+    g = _grid(500)
+    ls, rp, ci = _linear(g, cupf.CustomPrecision.FP32, autotune=True)
+    A, b = _systems(rp, ci, 64, 7, torch.float32)
+    ls.setup(64)
+    ls.factorize(A)
+    want = ls.solve(b)
+    assert ls.plan_array("factor_tuned_launches")[1] == ls.plan_array("factor_level_warps").size > 0
+    ls.factorize_static_scratch(A)
+    assert torch.equal(ls.solve(b), want)
+
+
 @pytest.mark.parametrize("first,second", [(470, 479), (479, 470)])
 def test_one_padded_batch_has_one_class(first, second):
     """500 buses are 420 fronts: 420 x 476 systems is where class 2 begins, and

@@ -343,3 +343,16 @@ def test_tasks_give_the_level_kernels_factors(batch, policy):
         V0 = torch.tensor(g.flat_start(batch), device="cuda")
         out.append(s.solve_batch_device(S, V0, config=cupf.NRConfig(tolerance=1e-12, max_iter=2))[0])
     assert torch.equal(out[0], out[1])
+
+
+def test_task_arrays_have_exact_names():
+    """Names of plan arrays are not prefixes, and a class is one of 0 to 3."""
+    g = G.make_grid(60, 90, 12, seed=1060)
+    s = cupf.NewtonSolver(cupf.NewtonOptions(backend=cupf.BackendKind.CUDA))
+    s.analyze_host(g.indptr, g.indices, g.n_bus, g.pv, g.pq)
+    for name in ("task_meta", "task_meta:3", "task_words:0", "task_sweep_stages:1"):
+        assert s.plan_array(name).size
+    assert s.plan_array("task_class").tolist() == [-1] and s.plan_array("task_classes").size == 0
+    for name in ("task_metadata", "task_stages_", "task_sweep_", "task_words:4", "task_words:", "task_words:0x"):
+        with pytest.raises(Exception):
+            s.plan_array(name)
