@@ -379,16 +379,21 @@ __global__ void k_load_features(const double* __restrict__ sbus, long long sbus_
 
 // mean-squared-error gradient on the first n_out columns:
 // g = 2 (pred - target) / (B n_out) in bf16 (0 in padding), loss += sum (pred - target)^2 / (B n_out)
-// A warp takes rows of the batch (no index division), and a block adds its
-// part of the loss with one atomic: one per warp and row would queue on the
-// single address.
+// A warp takes rows of the batch (no index division).  A lane's 16 squares of a
+// chunk are summed in FP32, everything above in FP64: FP32 atomics left the
+// loss with errors of 1e-6 that changed from run to run.  With parts, each block
+// leaves its share of the loss there, and the column sums that follow in a
+// training step add the shares in block order beside their own work (a last
+// block that added them here took 3 us of a step's 600); without, a block adds
+// its share to the loss with one FP32 atomic.
+constexpr int kMseBlocks = 148 * 8;
 __global__ void __launch_bounds__(256)
     k_mse_grad(const float* __restrict__ pred, int ld, const float* __restrict__ target, int n_out, int B,
-               __nv_bfloat16* __restrict__ grad, float* __restrict__ loss) {
-  __shared__ float part[8];
+               __nv_bfloat16* __restrict__ grad, float* __restrict__ loss, double* __restrict__ parts) {
+  __shared__ double part[8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float scale = 1.0f / ((float)B * (float)n_out);
-  float local = 0.0f;
+  double local = 0.0;
   // (row, 512-column chunk) pairs over the warps
   const int chunks = (ld + 511) / 512;
   for (long long i = (long long)blockIdx.x * 8 + warp; i < (long long)B * chunks; i += (long long)gridDim.x * 8) {
@@ -397,34 +402,56 @@ __global__ void __launch_bounds__(256)
     const float* p = pred + b * ld;
     const float* y = target + b * n_out;
     __nv_bfloat16* g = grad + b * ld;
+    float sq = 0.0f;
 #pragma unroll 8
     for (int k = k0 + lane; k < k1; k += 32) {
       float gval = 0.0f;
       if (k < n_out) {
         const float d = p[k] - y[k];
         gval = 2.0f * d * scale;
-        local += d * d * scale;
+        sq += d * d;
       }
       g[k] = __float2bfloat16(gval);
     }
+    local += (double)sq;
   }
   for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
   if (lane == 0) part[warp] = local;
   __syncthreads();
-  if (threadIdx.x == 0 && loss) {
+  if (threadIdx.x == 0) {
     for (int w = 1; w < 8; ++w) local += part[w];
-    atomicAdd(loss, local);
+    if (B > 0 && n_out > 0) local /= (double)B * (double)n_out;
+    if (parts) parts[blockIdx.x] = local;
+    else if (loss) atomicAdd(loss, (float)local);
   }
 }
 
 // column sums of a bf16 [rows][cols] matrix into fp32 [cols]
 // (a block per 32 columns, its 32 warps share the rows; the partial sums are
 // added in warp order.  One thread per column walking all rows was a chain of
-// `rows` dependent loads on cols / 256 blocks.)
+// `rows` dependent loads on cols / 256 blocks.  An element passes through at
+// most rows / 32 + 31 additions instead of `rows`, which is what bounds the
+// rounding error; summing in FP64 instead cost the training step of 2,000
+// buses x 1,024 3 us of 598.)
+// parts: one more block adds n_parts FP64 values to *acc, in a fixed order.
 __global__ void __launch_bounds__(1024)
-    k_col_sum_bf16(const __nv_bfloat16* __restrict__ g, int rows, int cols, float* __restrict__ out) {
+    k_col_sum_bf16(const __nv_bfloat16* __restrict__ g, int rows, int cols, float* __restrict__ out,
+                   const double* __restrict__ parts, int n_parts, float* __restrict__ acc) {
   __shared__ float part[32][33];
   const int lane = threadIdx.x, warp = threadIdx.y;
+  if (parts && blockIdx.x == gridDim.x - 1) {
+    __shared__ double sum[32];
+    double s = 0.0;
+    for (int i = warp * 32 + lane; i < n_parts; i += 1024) s += parts[i];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) sum[warp] = s;
+    __syncthreads();
+    if (warp == 0 && lane == 0) {
+      for (int w = 1; w < 32; ++w) s += sum[w];
+      *acc = (float)((double)*acc + s);
+    }
+    return;
+  }
   const int c = blockIdx.x * 32 + lane;
   float s = 0.0f;
   if (c < cols) {
@@ -736,15 +763,35 @@ int mlp_load_features(const double* sbus, long long sbus_stride, const double* s
 int mlp_mse_grad(const float* pred, int ld, const float* target, int n_out, int B, void* grad, float* loss,
                  void* stream) {
   return guarded([&] {
-    k_mse_grad<<<kSMs * 8, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        pred, ld, target, n_out, B, static_cast<__nv_bfloat16*>(grad), loss);
+    k_mse_grad<<<kMseBlocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        pred, ld, target, n_out, B, static_cast<__nv_bfloat16*>(grad), loss, nullptr);
+  });
+}
+
+int mlp_mse_parts(void) { return kMseBlocks; }
+
+int mlp_mse_grad_parts(const float* pred, int ld, const float* target, int n_out, int B, void* grad, double* parts,
+                       void* stream) {
+  return guarded([&] {
+    if (!parts) throw std::invalid_argument("mlp_mse_grad_parts: parts must not be null");
+    k_mse_grad<<<kMseBlocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        pred, ld, target, n_out, B, static_cast<__nv_bfloat16*>(grad), nullptr, parts);
   });
 }
 
 int mlp_col_sum_bf16(const void* g, int rows, int cols, float* out, void* stream) {
   return guarded([&] {
     k_col_sum_bf16<<<(cols + 31) / 32, dim3(32, 32), 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(g), rows, cols, out);
+        static_cast<const __nv_bfloat16*>(g), rows, cols, out, nullptr, 0, nullptr);
+  });
+}
+
+int mlp_col_sum_bf16_parts(const void* g, int rows, int cols, float* out, const double* parts, int n_parts, float* acc,
+                           void* stream) {
+  return guarded([&] {
+    if (!parts || n_parts < 0 || !acc) throw std::invalid_argument("mlp_col_sum_bf16_parts: parts and acc must not be null");
+    k_col_sum_bf16<<<(cols + 31) / 32 + 1, dim3(32, 32), 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const __nv_bfloat16*>(g), rows, cols, out, parts, n_parts, acc);
   });
 }
 

@@ -72,7 +72,7 @@ EXPORTS = [
 # exported symbols of include/cupf_mlp.h (warm-start network kernels)
 MLP_EXPORTS = [
     "mlp_last_error", "mlp_gemm_bf16", "mlp_error_flag", "mlp_set_wait_test", "mlp_transpose_bf16", "mlp_standardize",
-    "mlp_mse_grad",
+    "mlp_mse_grad", "mlp_mse_grad_parts", "mlp_mse_parts", "mlp_col_sum_bf16_parts",
     "mlp_col_sum_bf16", "mlp_adam", "mlp_load_features", "mlp_gemm_bf16_split",
     "mlp_gram_f64", "mlp_cholesky_solve_f64", "mlp_refit_last_error",
 ]
@@ -148,6 +148,9 @@ def _declare(lib: C.CDLL) -> None:
         "mlp_standardize": ([_vp, _vp, _vp, _vp, _i64, _i32, _i32, _i32, _vp], _i32),
         "mlp_load_features": ([_vp, _i64, _vp, _vp, _i32, _i32, _vp, _vp, _vp, _i64, _i32, _i32, _i32, _vp], _i32),
         "mlp_mse_grad": ([_vp, _i32, _vp, _i32, _i32, _vp, _vp, _vp], _i32),
+        "mlp_mse_grad_parts": ([_vp, _i32, _vp, _i32, _i32, _vp, _vp, _vp], _i32),
+        "mlp_mse_parts": ([], _i32),
+        "mlp_col_sum_bf16_parts": ([_vp, _i32, _i32, _vp, _vp, _i32, _vp, _vp], _i32),
         "mlp_col_sum_bf16": ([_vp, _i32, _i32, _vp, _vp], _i32),
         "mlp_adam": ([_vp, _vp, _vp, _vp, _vp, _i64, C.c_float, C.c_float, C.c_float, C.c_float, _i32, C.c_float,
                       _vp], _i32),

@@ -175,7 +175,8 @@ class MLP:
                  "actT": t.empty(max(self.dims_in), B, dtype=bf, device=d),
                  "gW": [t.empty(self.dims_out[i], self.dims_in[i], device=d) for i in range(L + 1)],
                  "gb": [t.empty(self.dims_out[i], device=d) for i in range(L + 1)],
-                 "loss": t.zeros(1, device=d)}
+                 "loss": t.zeros(1, device=d),
+                 "loss_parts": t.empty(self.lib.mlp_mse_parts(), dtype=t.float64, device=d)}
             self._bufs[key] = h
         return self._bufs[key]
 
@@ -214,8 +215,9 @@ class MLP:
         """Gradients of the mean-squared error against target (fp32 [B, n_out])
         into h['gW'] / h['gb']; the loss accumulates into h['loss']."""
         B = h["p"].shape[0]
-        self._check(self.lib.mlp_mse_grad(_ptr(h["p"]), self.no, _ptr(target), self.n_out, B, _ptr(h["gp"]),
-                                          _ptr(h["loss"]), self._stream()))
+        parts = h["loss_parts"]
+        self._check(self.lib.mlp_mse_grad_parts(_ptr(h["p"]), self.no, _ptr(target), self.n_out, B, _ptr(h["gp"]),
+                                                _ptr(parts), self._stream()))
         g = h["gp"]
         H = self.hidden
         for i in range(self.layers, -1, -1):
@@ -226,7 +228,11 @@ class MLP:
             self.transpose(g, gT)
             self.transpose(act, actT)
             self.gemm(gT, actT, h["gW"][i], EPI_F32)                    # dW = g^T act
-            self._check(self.lib.mlp_col_sum_bf16(_ptr(g), B, d_out, _ptr(h["gb"][i]), self._stream()))
+            if i == self.layers:  # adds the parts of the loss as well
+                self._check(self.lib.mlp_col_sum_bf16_parts(_ptr(g), B, d_out, _ptr(h["gb"][i]), _ptr(parts),
+                                                            parts.numel(), _ptr(h["loss"]), self._stream()))
+            else:
+                self._check(self.lib.mlp_col_sum_bf16(_ptr(g), B, d_out, _ptr(h["gb"][i]), self._stream()))
             if i > 0:
                 gn = h["g"][i % 2]
                 # (g W)[:, hidden part] * gelu'(z): the rows of W^T that multiply a_{i-1}

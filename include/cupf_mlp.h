@@ -84,11 +84,21 @@ int mlp_load_features(const double* sbus, long long sbus_stride, const double* s
                       int n_extra, const float* mean, const float* inv_std, void* x, long long ldx, int B, int rows,
                       int width, void* stream);
 /* Mean-squared error on the first n_out of ld columns: grad (bf16 [B][ld]) and
- * *loss += mean squared difference (fp32, may be NULL). */
+ * *loss += mean squared difference (fp32, may be NULL; the blocks' parts are
+ * added by atomics, so its last bits can vary). */
 int mlp_mse_grad(const float* pred, int ld, const float* target, int n_out, int B, void* grad, float* loss,
                  void* stream);
+/* The same gradient; the mean squared difference is left in parts as
+ * mlp_mse_parts() FP64 shares, to be added by mlp_col_sum_bf16_parts. */
+int mlp_mse_grad_parts(const float* pred, int ld, const float* target, int n_out, int B, void* grad, double* parts,
+                       void* stream);
+int mlp_mse_parts(void);
 /* out[c] = sum_r g[r][c] (g bf16 [rows][cols], out fp32). */
 int mlp_col_sum_bf16(const void* g, int rows, int cols, float* out, void* stream);
+/* The same, and *acc += sum of parts[0 .. n_parts), added in FP64 in a fixed
+ * order (the training step's loss, which then repeats bit for bit). */
+int mlp_col_sum_bf16_parts(const void* g, int rows, int cols, float* out, const double* parts, int n_parts, float* acc,
+                           void* stream);
 /* Adam step on fp32 master weights w (n elements) with moments m, v; writes
  * the bf16 copy w_bf16 when not NULL.  step counts from 1. */
 int mlp_adam(float* w, const float* grad, float* m, float* v, void* w_bf16, long long n, float lr, float b1, float b2,

@@ -618,3 +618,48 @@ def test_warm_start_checkpoint_round_trip(torch, tmp_path):
     other = WarmStart(g, hidden=256, layers=2, seed=0)
     with pytest.raises(ValueError):
         other.load(path)
+
+
+@pytest.mark.parametrize("B,n_out,ld", [(1, 1, 128), (128, 300, 384), (1000, 513, 640), (1024, 3573, 3584)])
+def test_training_sums_keep_their_precision_and_repeat(torch, B, n_out, ld):
+    """The loss is an FP64 sum of FP32 sums of at most 16 squares: at most 17
+    roundings of 2^-24 on the way to it (the square, 15 additions, the result)
+    and one for the addition to what the loss holds, whatever the batch; and
+    the same bits in every call.  Large and small rows together, so
+    that an FP32 running sum would lose the small ones.  The bias gradients are
+    FP32 sums of 32 interleaved parts: at most ceil(B / 32) + 31 roundings,
+    each of at most 2^-24 of the sum of magnitudes."""
+    from cupf import _capi
+    from cupf.warm_start import _ptr
+
+    lib = _capi.load()
+    g = torch.Generator(device="cuda").manual_seed(B + n_out)
+    row = 10.0 ** (2 * torch.rand(B, 1, device="cuda", generator=g) - 1)
+    pred = row * torch.randn(B, ld, device="cuda", generator=g)
+    target = torch.randn(B, n_out, device="cuda", generator=g)
+    d = (pred[:, :n_out] - target).double()
+    want = float((d * d).sum() / (B * n_out))
+    parts = torch.empty(lib.mlp_mse_parts(), dtype=torch.float64, device="cuda")
+    gb, losses, sums, stream = torch.empty(ld, device="cuda"), [], [], torch.cuda.current_stream().cuda_stream
+    for ordered in (True, True, True, False):
+        grad = torch.empty(B, ld, dtype=torch.bfloat16, device="cuda")
+        loss = torch.zeros(1, device="cuda")
+        if ordered:
+            assert lib.mlp_mse_grad_parts(_ptr(pred), ld, _ptr(target), n_out, B, _ptr(grad), _ptr(parts), stream) == 0
+            assert lib.mlp_col_sum_bf16_parts(_ptr(grad), B, ld, _ptr(gb), _ptr(parts), parts.numel(), _ptr(loss),
+                                              stream) == 0
+        else:
+            assert lib.mlp_mse_grad(_ptr(pred), ld, _ptr(target), n_out, B, _ptr(grad), _ptr(loss), stream) == 0
+            assert lib.mlp_col_sum_bf16(_ptr(grad), B, ld, _ptr(gb), stream) == 0
+        losses.append(float(loss))
+        sums.append(gb.clone())
+    assert losses[0] == losses[1] == losses[2] and abs(losses[0] - want) <= 18 * 2.0 ** -24 * want
+    # (the parts added by FP32 atomics, each addition off by at most 2^-24 of the sum)
+    assert abs(losses[3] - want) <= (17 + parts.numel()) * 2.0 ** -24 * want
+    assert all(torch.equal(v, sums[0]) for v in sums)
+    exact = 2.0 * d / (B * n_out)
+    assert float((grad[:, :n_out].double() - exact).abs().max()) <= 2.0 ** -8 * float(exact.abs().max())
+    assert not grad[:, n_out:].any()
+    s = grad.double().sum(0)
+    bound = (-(-B // 32) + 31) * 2.0 ** -24 * grad.double().abs().sum(0)
+    assert bool(((gb.double() - s).abs() <= bound).all())
