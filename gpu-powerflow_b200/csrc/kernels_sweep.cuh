@@ -366,9 +366,17 @@ void launch_sweep_stage(int mode, const SweepTaskStage& st, const SweepTaskArgs<
       else launch_sweep_tasks<M, T, 1, 1, 1>(st, a, groups, meta, words, lanes, s);
       return;
     }
-    if (st.warps > 1) launch_sweep_tasks<M, T, 1, sizeof(T) == 8 ? 4 : 8, 2>(st, a, groups, meta, words, lanes, s);
-    else if (st.lanes == 16) launch_sweep_tasks<M, T, 1, 16, 1>(st, a, groups, meta, words, lanes, s);
-    else launch_sweep_tasks<M, T, 1, 8, 1>(st, a, groups, meta, words, lanes, s);
+    // the shapes sweep_task_specs uses (block teams take 4 scenarios in FP64:
+    // the specs' limits fill shared memory with 4 x 8 and 8 x 4 bytes alike)
+    if (st.warps == 2 && st.lanes == 8 && st.pack == 1)
+      launch_sweep_tasks<M, T, 1, sizeof(T) == 8 ? 4 : 8, 2>(st, a, groups, meta, words, lanes, s);
+    else if (st.warps == 1 && st.lanes == 16 && st.pack == 1)
+      launch_sweep_tasks<M, T, 1, 16, 1>(st, a, groups, meta, words, lanes, s);
+    else if (st.warps == 1 && st.lanes == 8 && st.pack == 1)
+      launch_sweep_tasks<M, T, 1, 8, 1>(st, a, groups, meta, words, lanes, s);
+    else
+      throw std::runtime_error("sweep tasks: no kernel for teams of " + std::to_string(st.warps) + " warps, " +
+                               std::to_string(st.lanes) + " lanes, " + std::to_string(st.pack) + " scenarios a lane");
   };
   switch (mode) {
     case kSweepL: run(std::integral_constant<SweepMode, kSweepL>{}); break;

@@ -686,19 +686,22 @@ void launch_factor_stage(const TaskStage& st, const FactorArgs<T, T>& a, const i
     else launch_tasks<T, 1, 1, 1>(st, a, meta, words, lanes, s);
     return;
   }
-  switch (10 * st.warps + st.pack) {  // (the shapes factor_task_specs uses)
-    case 12: launch_tasks<T, 2, 8, 1>(st, a, meta, words, lanes, s); break;
-    case 14:
-      if constexpr (sizeof(T) == 4) launch_tasks<T, 4, 8, 1>(st, a, meta, words, lanes, s);
-      break;
-    case 21: launch_tasks<T, 1, 8, 2>(st, a, meta, words, lanes, s); break;
-    case 22:
-      if constexpr (sizeof(T) == 4) launch_tasks<T, 2, 8, 2>(st, a, meta, words, lanes, s);
-      break;
-    case 41: launch_tasks<T, 1, 8, 4>(st, a, meta, words, lanes, s); break;
-    case 81: launch_tasks<T, 1, sizeof(T) == 8 ? 4 : 8, 8>(st, a, meta, words, lanes, s); break;
-    default: launch_tasks<T, 1, 8, 1>(st, a, meta, words, lanes, s); break;
+  const auto is = [&](int warps, int lanes_, int pack) {
+    return st.warps == warps && st.lanes == lanes_ && st.pack == pack;
+  };
+  constexpr int kTopLanes = sizeof(T) == 8 ? 4 : 8;
+  // the shapes factor_task_specs uses; any other would leave its fronts unfactored
+  if (is(1, 8, 1)) return launch_tasks<T, 1, 8, 1>(st, a, meta, words, lanes, s);
+  if (is(1, 8, 2)) return launch_tasks<T, 2, 8, 1>(st, a, meta, words, lanes, s);
+  if (is(2, 8, 1)) return launch_tasks<T, 1, 8, 2>(st, a, meta, words, lanes, s);
+  if (is(4, 8, 1)) return launch_tasks<T, 1, 8, 4>(st, a, meta, words, lanes, s);
+  if (is(8, kTopLanes, 1)) return launch_tasks<T, 1, kTopLanes, 8>(st, a, meta, words, lanes, s);
+  if constexpr (sizeof(T) == 4) {
+    if (is(1, 8, 4)) return launch_tasks<T, 4, 8, 1>(st, a, meta, words, lanes, s);
+    if (is(2, 8, 2)) return launch_tasks<T, 2, 8, 2>(st, a, meta, words, lanes, s);
   }
+  throw std::runtime_error("factor tasks: no kernel for teams of " + std::to_string(st.warps) + " warps, " +
+                           std::to_string(st.lanes) + " lanes, " + std::to_string(st.pack) + " scenarios a lane");
 }
 
 }  // namespace cupf_b200

@@ -573,6 +573,7 @@ TaskPlan build_task_plan(const FactorProgram& fp, int front_limit, const std::ve
   std::vector<uint8_t> out(fp.P, 0);  // left to the level launches
   std::vector<int32_t> scratch;
   for (int32_t p = 0; p < fp.P; ++p) {
+    if (fp.nc[p] > 8) return none;  // (the kernels' pivot blocks have up to 8 columns)
     const double fs = fp.fsz[p], nc = fp.nc[p], uc = fs - nc;
     sh.work[p] = 60 + fs * (fs + 1) + uc * (uc + 1) * (2 + nc) / 2;
     for (int32_t fr = fp.front_ptr[p]; fr < fp.front_ptr[p + 1]; ++fr)
