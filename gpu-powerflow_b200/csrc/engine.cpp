@@ -478,6 +478,9 @@ void Engine::prepare_tasks(int32_t B) {
   std::vector<int> classes{task_class(fp_.P, 1)};
   if (B > 1)  // (the classes of larger batches follow one another)
     for (int c = task_class(fp_.P, kWarp); c <= task_class(fp_.P, B); ++c) classes.push_back(c);
+  // wide_min_front = 1 asks for the general kernels: every front on the
+  // any-size tier, and the sweeps level by level
+  if (cfg_.wide_min_front == 1) classes.clear();
   for (int cls : classes) {
     if (fp_.P >= kTaskFronts && !d.task_sets.count(cls)) {
       auto ts = std::make_unique<TaskSet>();

@@ -85,7 +85,8 @@ typedef struct {
   int32_t parallel_nd_base_large; /* than 20,000 vertices / otherwise; 0 = the defaults 4, 4000, 20000 */
   int32_t wide_min_front;       /* factor launches whose largest front has at least this many rows run the
                                    wide tier, which takes fronts of any size (the register kernels stop at
-                                   64 rows); 1..65, 0 = 65.  Both give the same factors. */
+                                   64 rows); 1..65, 0 = 65.  Both give the same factors.  1 leaves nothing to
+                                   the subtree tasks: the general kernels throughout, the sweeps by levels */
   int32_t tc_min_front;         /* precision TF32: launches whose largest front has at least this many rows
                                    run their trailing update CB = A22 - L21 U12 on the tensor cores
                                    (tcgen05 kind::tf32, operands split hi + lo, fp32 accumulation); 0 = 65,

@@ -246,3 +246,61 @@ def test_launches_beside_tasks_fit_the_front_scratch():
         M = sp.csr_matrix((vals[k], A.indices, A.indptr), shape=(n, n))
         # diagonally dominant: growth below 2, n = 28 rows to a block
         assert np.linalg.norm(M @ x[k] - b[k]) <= 1e-13 * np.linalg.norm(b[k])
+
+
+# batches of every class on 2,000 buses (1,671 fronts): a single system, little
+# (up to 128), medium, and from 480 systems on much work; odd ones among them
+@pytest.mark.parametrize("batch,cls", [(1, 0), (2, 1), (33, 1), (128, 1), (161, 2), (449, 3), (517, 3)])
+@pytest.mark.parametrize("precision", [cupf.CustomPrecision.FP64, cupf.CustomPrecision.FP32])
+def test_tasks_solve_like_the_general_kernels(precision, batch, cls):
+    """Factor, solve and transpose solve by subtree tasks against the general
+    kernels (wide_min_front = 1: the any-size tier and the level sweeps): the
+    same solutions, bit for bit."""
+    import torch
+
+    g = _grid(2000)
+    dtype = torch.float64 if precision == cupf.CustomPrecision.FP64 else torch.float32
+    out = []
+    for wide in (0, 1):
+        ls, rp, ci = _linear(g, precision, autotune=False, wide_min_front=wide)
+        A, b = _systems(rp, ci, batch, batch, dtype)
+        ls.setup(batch)
+        ls.factorize(A)
+        assert ls.plan_array("task_class")[0] == (-1 if wide else cls)
+        out.append((ls.solve(b), ls.solve_transpose(b)))
+        assert not ls.singular_flags().any()
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+    # and they solve the systems: diagonally dominant rows, so to a few hundred
+    # times the unit roundoff
+    if batch <= 33:
+        rows = torch.tensor(np.repeat(np.arange(rp.size - 1), np.diff(rp)), device="cuda")
+        cols = torch.tensor(ci.astype(np.int64), device="cuda")
+        eps = torch.finfo(dtype).eps
+        for x, r, c in ((out[0][0], rows, cols), (out[0][1], cols, rows)):
+            y = torch.zeros_like(b).index_add_(1, r, A.double() * x.double()[:, c])
+            assert float((y - b).norm() / b.norm()) <= 300 * eps
+
+
+@pytest.mark.parametrize("batch,cls", [(1, 0), (31, 1), (161, 2), (517, 3)])
+@pytest.mark.parametrize("policy", ["FP64", "Mixed", "FP32"])
+def test_newton_and_gradients_of_every_class_keep_the_general_kernels_bits(policy, batch, cls):
+    """Two Newton updates, and the gradients at the state they reach, against
+    the general kernels."""
+    import torch
+
+    g = _grid(2000)
+    S, V0 = g.scenarios(batch, seed=batch), g.flat_start(batch)
+    grads = np.random.default_rng(batch).standard_normal((2, batch, g.n_bus))
+    out = []
+    for wide in (0, 1):
+        s = _newton(g, policy, autotune=False, wide_min_front=wide)
+        so = cupf.SolveOptions(prepare_adjoint_cache=policy != "FP32")  # (the adjoint needs an FP64 state)
+        r = s.solve_batch(g.indptr, g.indices, g.data, g.n_bus, g.n_bus, S, V0, g.pv, g.pq,
+                          cupf.NRConfig(tolerance=1e-12, max_iter=2), so)
+        assert s.plan_array("task_class")[0] == (-1 if wide else cls)
+        out.append([r.V_numpy])
+        if policy != "FP32":
+            a = s.solve_adjoint(*grads, g.pv, g.pq)
+            out[-1] += [a.lambda_numpy, a.grad_load_p_numpy, a.grad_load_q_numpy]
+    for a, b in zip(*out):
+        assert np.isfinite(a).all() and np.array_equal(a, b)
