@@ -249,19 +249,8 @@ bool Engine::tf32_factors() const { return cfg_.factor_precision == kFactorTF32 
 
 bool Engine::single_system() const { return cfg_.batch1_schedule == 0 && d_->B == 1; }
 
-// Small trees are a few short levels, and the stages' launches cost as much
-// as the levels': per graph-mode iteration 94 against 113 us by levels and
-// by tasks with 100 buses (about 75 fronts) x 64, 127 against 126 us with
-// 300 buses (about 250 fronts), 220 against 185 us with 1,000.
-constexpr int kTaskFronts = 300;
-// Small trees sweep level by level: factorize + solve + transpose solve with
-// 300 buses (about 250 fronts) x 20 takes 321 us by levels and 349 us by
-// tasks, 610 and 696 us x 1,500 in FP64; 500 buses (420 fronts) x 200 515 and
-// 448 us, 800 buses x 300 635 and 532 us.
-constexpr int kSweepTaskFronts = 400;
-
 bool Engine::use_tasks() const {
-  if (!d_->ts || d_->ts->tasks.stages.empty() || (d_->B == 1 && cfg_.batch1_schedule == 1)) return false;
+  if (!d_->ts || (d_->B == 1 && cfg_.batch1_schedule == 1)) return false;
   // for a single system the other way is one launch over the whole tree
   return !(single_system() && !d_->ts->rest.empty());
 }
@@ -481,13 +470,16 @@ void Engine::prepare_tasks(int32_t B) {
   // wide_min_front = 1 asks for the general kernels: every front on the
   // any-size tier, and the sweeps level by level
   if (cfg_.wide_min_front == 1) classes.clear();
+  const int elem = factor_is_double() ? 8 : 4;
   for (int cls : classes) {
     if (fp_.P >= kTaskFronts && !d.task_sets.count(cls)) {
       auto ts = std::make_unique<TaskSet>();
       ts->tasks = task_plan(cls);
-      ts->meta.upload(ts->tasks.meta);
-      ts->words.upload(ts->tasks.words);
-      if (!ts->tasks.stages.empty()) {
+      // (what a single system does not use is not uploaded; larger batches of
+      // one class differ)
+      if (!ts->tasks.stages.empty() && (cls > 0 || tasks_pay(ts->tasks, fp_.P, 1, elem))) {
+        ts->meta.upload(ts->tasks.meta);
+        ts->words.upload(ts->tasks.words);
         // the fronts no task covers, level by level
         std::vector<std::vector<int32_t>> by_level(fp_.num_levels);
         std::vector<int32_t> order, qof(fp_.P), meta;
@@ -504,6 +496,8 @@ void Engine::prepare_tasks(int32_t B) {
                       fp_.front_meta.begin() + (size_t)(qof[p] + 1) * kFrontMetaInts);
         ts->rest_meta.upload(meta);
         pad_lists(ts->rest, order, ts->rest_src, ts->rest_dst);
+      } else {
+        ts->tasks = TaskPlan();  // planned, and of no use
       }
       d.task_sets[cls] = std::move(ts);
       assign_tiers(tc_min_);
@@ -519,15 +513,17 @@ void Engine::prepare_tasks(int32_t B) {
   }
 }
 
-// Makes the current batch's plans the ones in use.
+// Makes the current batch's plans the ones in use, where they pay.
 void Engine::select_tasks() {
   auto& d = *d_;
   // by the padded batch, which the captured solve and the tuned shapes go by too
-  const int cls = task_class(fp_.P, d.B == 1 ? 1 : d.Bp);
+  const int batch = d.B == 1 ? 1 : d.Bp, cls = task_class(fp_.P, batch), elem = factor_is_double() ? 8 : 4;
   const auto ts = d.task_sets.find(cls);
   const auto ss = d.sweep_sets.find(sweep_class(cls));
-  d.ts = ts == d.task_sets.end() ? nullptr : ts->second.get();
-  d.sweeps = ss == d.sweep_sets.end() ? nullptr : ss->second.get();
+  d.ts = ts != d.task_sets.end() && tasks_pay(ts->second->tasks, fp_.P, batch, elem) ? ts->second.get() : nullptr;
+  d.sweeps = ss != d.sweep_sets.end() && sweep_tasks_pay(ss->second->plan, fp_.P, fp_.num_levels, batch, elem)
+                 ? ss->second.get()
+                 : nullptr;
 }
 
 // Source lists in launch order, each padded to its launch's longest.
@@ -1172,7 +1168,12 @@ bool Engine::task_array(std::string name, std::vector<int32_t>* out) const {
     return true;
   }
   if (name == "task_classes") {
-    for (const auto& s : d_->task_sets) out->push_back(s.first);
+    for (const auto& s : d_->task_sets)
+      if (!s.second->tasks.stages.empty()) out->push_back(s.first);
+    return true;
+  }
+  if (name == "task_sweeps") {
+    out->push_back(use_sweep_tasks() ? 1 : 0);
     return true;
   }
   int cls = 3;  // "name:class"
@@ -1311,7 +1312,7 @@ void Engine::backward_all(cudaStream_t s) {
   stage_end(3, s);
 }
 
-bool Engine::use_sweep_tasks() const { return d_->sweeps && !d_->sweeps->plan.stages.empty(); }
+bool Engine::use_sweep_tasks() const { return d_->sweeps != nullptr; }
 
 // One sweep over the subtree tasks (modes: launch_sweep_stage), a launch per stage.
 template <typename T>

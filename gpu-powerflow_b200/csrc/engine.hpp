@@ -134,7 +134,8 @@ class Engine {
   // a team); the sweeps': "task_sweep_meta", "task_sweep_words",
   // "task_sweep_stages"; ":c" after a name picks the batch class (default 3);
   // "task_classes": the classes whose factorization plans are on the device;
-  // "task_class": the class whose tasks factor the current batch, -1 when none do
+  // "task_class": the class whose tasks factor the current batch, -1 when none do;
+  // "task_sweeps": 1 when tasks sweep it
   // (false: no such name)
   bool task_array(std::string name, std::vector<int32_t>* out) const;
   int32_t tc_threshold() const { return tc_min_; }

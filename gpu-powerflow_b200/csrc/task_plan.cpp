@@ -563,8 +563,50 @@ std::vector<TaskStageSpec> sweep_task_specs(int cls) {
   return {{500, 0, 160, 4000, 150, 1, 8, 1}, {2500, 0, 2400, 11000, 640, 2, 8, 1}, {0, 0, 2400, 11000, 640, 2, 8, 1}};
 }
 
+// Small trees are a few short levels, and the stages' launches cost as much as
+// the levels': per graph-mode iteration 94 us by levels and 113 by tasks
+// with 100 buses (about 75 fronts) x 64, 127 and 126 with 300 buses (about 250
+// fronts), 220 and 185 with 1,000.
+//
+// With few systems the time goes by what has to happen one after the other,
+// not by the work, and a stage with one long task is slower than the levels it
+// replaces.  The line for a single system, against the one launch over the
+// tree, is fitted (in us) to Newton solves of 214 random grids of 300 to 9,000
+// fronts, with a standard deviation of 6 us about it: the rule's choice is within
+// 0.4 % of the faster one on average below 1,400 fronts, where tasks
+// always lose 2 % (FP32) and 4 % (FP64), up to 26 %.  500 buses (420
+// fronts), one FP64 update: 138 us over the tree, 151 us by tasks; 700 buses
+// (589 fronts): 177 and 159.  For 2 to 32 systems only a heaviest chain of more
+// than about twice the tree's loses to the levels: 480 buses (408 fronts) x 2
+// 135 us by levels, 142 by tasks (FP32); 600 (498 fronts) 186 and 158.
+bool tasks_pay(const TaskPlan& tp, int fronts, int batch, int elem_bytes) {
+  if (fronts < kTaskFronts || tp.stages.empty()) return false;
+  if (fronts >= 2500) return true;
+  if (batch == 1)
+    return 1.3 * tp.chain + 0.002 * tp.chain_work + (elem_bytes == 8 ? 16 : 13) <
+           2.2 * tp.path + 0.0083 * tp.path_work + 3.0 * tp.stages.size();
+  return !(batch <= 32 && fronts < 1200 && tp.chain_work > 2.15 * tp.path_work);
+}
+
+// The same for the sweeps, whose task works one front after the other: about
+// 1.5 us each, against 9 us a level; the more systems, the more a level costs.
+// Fitted to the same grids: within 0.7 % of the faster choice on average for
+// every batch from 1 to 512 systems, where tasks always lose 1 to 5.6 %.  Solve and
+// transpose solve, FP32: 480 buses (chain 49, 12 levels) x 2 256 us by levels
+// and 331 by tasks, x 2,048 548 and 462; 600 (chain 44, 15 levels) x 2
+// 335 and 322.  Trees of fewer than 400 fronts gain only from a batch
+// of a thousand (350 buses, 304 fronts, x 512 285 and 332, x 2,048 478 and 431).
+bool sweep_tasks_pay(const SweepPlan& sp, int fronts, int levels, int batch, int elem_bytes) {
+  if (fronts < kSweepTaskFronts || sp.stages.empty()) return false;
+  if (fronts >= 2500) return true;
+  const double items = (double)fronts * std::max(batch, 32);
+  if (items > 800e3) return true;  // (much work, whose stages are cut otherwise)
+  return sp.chain <= 6.4 * levels - 45 + items / (elem_bytes == 8 ? 30e3 : 45e3);
+}
+
 TaskPlan build_task_plan(const FactorProgram& fp, int front_limit, const std::vector<TaskStageSpec>& specs) {
-  const TaskPlan none{{}, {}, {}, std::vector<uint8_t>(fp.P, 0)};
+  TaskPlan none;
+  none.covered.assign(fp.P, 0);
   // element offsets and list lengths must fit the program's fields
   if (fp.u_total > INT32_MAX || fp.l_total > INT32_MAX || fp.cb_total > INT32_MAX || specs.empty()) return none;
   front_limit = std::min(front_limit, 128);
@@ -612,6 +654,9 @@ TaskPlan build_task_plan(const FactorProgram& fp, int front_limit, const std::ve
         st.warps = spec.warps;
         st.lanes = spec.lanes;
         st.pack = spec.pack;
+        // (the heaviest task comes first)
+        tp.chain += (int)tasks[0].order.size();
+        for (int32_t p : tasks[0].order) tp.chain_work += sh.work[p];
         for (const TaskBuild& t : tasks) {
           tp.meta.insert(tp.meta.end(), {(int32_t)tp.words.size(), t.words, (int32_t)t.order.size(), 0});
           write_task(sh, t, tp.words);
@@ -621,6 +666,15 @@ TaskPlan build_task_plan(const FactorProgram& fp, int front_limit, const std::ve
         tp.stages.push_back(st);
       });
   tp.covered = sh.done;
+  std::vector<int> depth(fp.P, 0);  // paths from the root down
+  std::vector<double> work(fp.P, 0.0);
+  for (int32_t p = fp.P - 1; p >= 0; --p) {
+    const int32_t par = fp.parent_panel[p];
+    depth[p] = 1 + (par >= 0 ? depth[par] : 0);
+    work[p] = sh.work[p] + (par >= 0 ? work[par] : 0.0);
+    tp.path = std::max(tp.path, depth[p]);
+    tp.path_work = std::max(tp.path_work, work[p]);
+  }
   return tp;
 }
 
@@ -661,6 +715,9 @@ SweepPlan build_sweep_plan(const FactorProgram& fp, const std::vector<TaskStageS
         st.warps = spec.warps;
         st.lanes = spec.lanes;
         st.pack = spec.pack;
+        size_t longest = 0;
+        for (const SweepBuild& t : tasks) longest = std::max(longest, t.order.size());
+        sp.chain += (int)longest;
         for (const SweepBuild& t : tasks) {
           sp.meta.insert(sp.meta.end(), {(int32_t)sp.words.size(), t.words, (int32_t)t.order.size(),
                                          (int32_t)t.ext_rows.size()});

@@ -56,6 +56,9 @@ struct TaskStageSpec {
   int pack = 1;        // ... and scenarios per lane
 };
 
+constexpr int kTaskFronts = 300;       // smallest trees that factor (sweep) as tasks: tasks_pay
+constexpr int kSweepTaskFronts = 400;
+
 // Classes of batches with stages of their own: 0 a single system; by the
 // fronts x systems of a batch, 1 little, 2 medium, 3 much work.
 int task_class(int fronts, int batch);
@@ -75,6 +78,11 @@ struct TaskPlan {
   std::vector<int32_t> words;
   std::vector<TaskStage> stages; // in launch order
   std::vector<uint8_t> covered;  // per panel: 1 when a task factors it
+  // What one factorization of few systems has to do one after the other, in
+  // fronts and in units of work: the heaviest task of every stage, and for
+  // comparison the longest path of the front tree.
+  int chain = 0, path = 0;
+  double chain_work = 0, path_work = 0;
   int tasks() const { return (int)(meta.size() / 4); }
 };
 
@@ -126,6 +134,7 @@ struct SweepPlan {
   std::vector<int32_t> meta;  // per task: program offset (words), words, fronts, external rows
   std::vector<int32_t> words;
   std::vector<SweepTaskStage> stages;  // leaves first
+  int chain = 0;  // fronts of the longest task of every stage
   int tasks() const { return (int)(meta.size() / 4); }
 };
 
@@ -140,5 +149,10 @@ SweepPlan build_sweep_plan(const FactorProgram& fp, const std::vector<TaskStageS
 // front that fits it is left; a front that does not fit it alone is left out
 // with its ancestors.  A pattern with repeated entries gives an empty plan.
 TaskPlan build_task_plan(const FactorProgram& fp, int front_limit, const std::vector<TaskStageSpec>& specs);
+
+// Whether a batch (1, or the batch padded to 32) factors faster by these tasks
+// than by the other schedules, and sweeps faster by tasks than level by level.
+bool tasks_pay(const TaskPlan& tp, int fronts, int batch, int elem_bytes);
+bool sweep_tasks_pay(const SweepPlan& sp, int fronts, int levels, int batch, int elem_bytes);
 
 }  // namespace cupf_b200

@@ -168,9 +168,9 @@ const char* cls_last_error(cls_handle h);
  * "tc_threshold" (one value: the front size from which TF32 factors use the
  * tensor cores, 0 for other precisions).  The factor_level arrays describe the
  * launches of the whole tree, which factor small trees and run in
- * cls_factorize_static_scratch.  Trees of 300 fronts and more otherwise factor
- * as subtree tasks ("task_class": the class of the current batch's tasks, -1
- * when none run; "task_classes": the classes planned on the device), and
+ * cls_factorize_static_scratch.  Trees of 300 fronts and more otherwise mostly
+ * factor as subtree tasks ("task_class": the class of the current batch's tasks, -1
+ * when none run; "task_sweeps": 1 when they sweep; "task_classes": the classes planned on the device), and
  * "factor_rest_warps", "factor_rest_tiers" and "factor_rest_placement" are the
  * same for the launches of the fronts that the tasks leave;
  * "factor_tuned_launches" counts the launches that the autotuner timed last (rest,

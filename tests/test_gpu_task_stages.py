@@ -193,7 +193,8 @@ def _systems(rp, ci, batch, seed, dtype):
 
 
 @pytest.mark.parametrize("precision", [cupf.CustomPrecision.FP64, cupf.CustomPrecision.FP32])
-@pytest.mark.parametrize("buses", [400, 500])  # 300 to 399 fronts: task factors under level sweeps; 400 and more
+# task factors under level sweeps (344 fronts); the tree launch under sweep tasks (420); tasks throughout
+@pytest.mark.parametrize("buses", [400, 500, 2000])
 def test_batch_of_one_sweeps_equal_the_lane_kernels(buses, precision):
     """Solve and transpose solve of a batch of one on the factors its tasks
     left in column 0, against the lane kernels' factors of every column
@@ -205,11 +206,12 @@ def test_batch_of_one_sweeps_equal_the_lane_kernels(buses, precision):
     out = []
     for schedule in (0, 1):
         ls, rp, ci = _linear(g, precision, batch1_schedule=schedule, autotune=False)
-        fronts = ls.plan_array("fp_fsz").size
-        assert (300 <= fronts < 400) if buses == 400 else fronts >= 400
         A, b = _systems(rp, ci, 1, 5, dtype)
         ls.setup(1)
         ls.factorize(A)
+        if schedule == 0:
+            assert (ls.plan_array("task_class")[0] >= 0) == (buses != 500)
+            assert ls.plan_array("task_sweeps")[0] == (buses != 400)
         out.append((ls.solve(b), ls.solve_transpose(b)))
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
 
@@ -304,3 +306,32 @@ def test_newton_and_gradients_of_every_class_keep_the_general_kernels_bits(polic
             out[-1] += [a.lambda_numpy, a.grad_load_p_numpy, a.grad_load_q_numpy]
     for a, b in zip(*out):
         assert np.isfinite(a).all() and np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("precision", [cupf.CustomPrecision.FP64, cupf.CustomPrecision.FP32])
+# buses, batch, factored by tasks, swept by tasks: trees on both sides of each
+# rule (tasks_pay, sweep_tasks_pay)
+@pytest.mark.parametrize("buses,batch,factor,sweep", [
+    (300, 64, False, False),   # 254 fronts
+    (500, 1, False, True),     # the tree launch is faster than a long chain of fronts
+    (700, 1, True, False),
+    (480, 2, False, False),    # a heaviest chain of more than twice the tree's longest path
+    (480, 33, True, False),    # one sweep task of 37 fronts, 12 levels
+    (600, 2, True, True),
+    (480, 2048, True, True),   # much work: the levels' cost grows with the batch, the chain's does not
+])
+def test_small_trees_take_the_faster_schedule_with_the_same_bits(buses, batch, factor, sweep, precision):
+    import torch
+
+    g = _grid(buses)
+    dtype = torch.float64 if precision == cupf.CustomPrecision.FP64 else torch.float32
+    out = []
+    for wide in (0, 1):
+        ls, rp, ci = _linear(g, precision, autotune=False, wide_min_front=wide)
+        A, b = _systems(rp, ci, batch, batch, dtype)
+        ls.setup(batch)
+        ls.factorize(A)
+        if not wide:
+            assert (ls.plan_array("task_class")[0] >= 0) == factor and ls.plan_array("task_sweeps")[0] == sweep
+        out.append((ls.solve(b), ls.solve_transpose(b)))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
