@@ -20,6 +20,7 @@
 #include <limits>
 #include <map>
 #include <memory>
+#include <set>
 #include <stdexcept>
 #include <string>
 
@@ -122,7 +123,7 @@ struct Engine::Impl {
       crow_child, crow_r, crow_src, crow_dst, asm_ptr, asm_local, perm, iperm, row_iperm, col_perm, level_fronts, fe_split, fe_dst, fe_src, front_meta;
   std::vector<LevelLaunch> levels;
   std::map<int, std::unique_ptr<TaskSet>> task_sets;    // by class
-  std::map<int, std::unique_ptr<SweepSet>> sweep_sets;  // by sweep_class(class)
+  std::map<int, std::unique_ptr<SweepSet>> sweep_sets;  // by sweep class
   TaskSet* ts = nullptr;                                // of the current batch (null: the level launches)
   SweepSet* sweeps = nullptr;
   void clear_tasks() {
@@ -464,13 +465,15 @@ SweepPlan Engine::sweep_plan(int cls) const {
 // classes take about as long as the symbolic analysis (2,000 buses: 15 ms).
 void Engine::prepare_tasks(int32_t B) {
   auto& d = *d_;
-  std::vector<int> classes{task_class(fp_.P, 1)};
-  if (B > 1)  // (the classes of larger batches follow one another)
-    for (int c = task_class(fp_.P, kWarp); c <= task_class(fp_.P, B); ++c) classes.push_back(c);
+  const int elem = factor_is_double() ? 8 : 4;
+  std::set<int> classes{task_class(fp_.P, 1, elem)}, sweeps{sweep_class(fp_.P, 1, elem)};
+  for (int32_t b = kWarp; b <= B; b += kWarp) {
+    classes.insert(task_class(fp_.P, b, elem));
+    sweeps.insert(sweep_class(fp_.P, b, elem));
+  }
   // wide_min_front = 1 asks for the general kernels: every front on the
   // any-size tier, and the sweeps level by level
-  if (cfg_.wide_min_front == 1) classes.clear();
-  const int elem = factor_is_double() ? 8 : 4;
+  if (cfg_.wide_min_front == 1) return;
   for (int cls : classes) {
     if (fp_.P >= kTaskFronts && !d.task_sets.count(cls)) {
       auto ts = std::make_unique<TaskSet>();
@@ -502,10 +505,11 @@ void Engine::prepare_tasks(int32_t B) {
       d.task_sets[cls] = std::move(ts);
       assign_tiers(tc_min_);
     }
-    const int sc = sweep_class(cls);
+  }
+  for (int sc : sweeps) {
     if (fp_.P >= kSweepTaskFronts && !d.sweep_sets.count(sc)) {
       auto ss = std::make_unique<SweepSet>();
-      ss->plan = sweep_plan(cls);
+      ss->plan = sweep_plan(sc);
       ss->meta.upload(ss->plan.meta);
       ss->words.upload(ss->plan.words);
       d.sweep_sets[sc] = std::move(ss);
@@ -517,9 +521,9 @@ void Engine::prepare_tasks(int32_t B) {
 void Engine::select_tasks() {
   auto& d = *d_;
   // by the padded batch, which the captured solve and the tuned shapes go by too
-  const int batch = d.B == 1 ? 1 : d.Bp, cls = task_class(fp_.P, batch), elem = factor_is_double() ? 8 : 4;
-  const auto ts = d.task_sets.find(cls);
-  const auto ss = d.sweep_sets.find(sweep_class(cls));
+  const int batch = d.B == 1 ? 1 : d.Bp, elem = factor_is_double() ? 8 : 4;
+  const auto ts = d.task_sets.find(task_class(fp_.P, batch, elem));
+  const auto ss = d.sweep_sets.find(sweep_class(fp_.P, batch, elem));
   d.ts = ts != d.task_sets.end() && tasks_pay(ts->second->tasks, fp_.P, batch, elem) ? ts->second.get() : nullptr;
   d.sweeps = ss != d.sweep_sets.end() && sweep_tasks_pay(ss->second->plan, fp_.P, fp_.num_levels, batch, elem)
                  ? ss->second.get()

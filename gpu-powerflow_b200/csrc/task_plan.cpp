@@ -521,14 +521,43 @@ int half_words(int64_t halves) { return (int)((halves + 1) / 2); }
 // takes 293 us (521 us with a launch per level; 408 us when the first stage
 // is followed by block teams only), the 10,000-bus grid x 64 209 us (540 us
 // per level; 315 us with subtrees of up to 2,500 units first).
-int task_class(int fronts, int batch) {
+//
+// The lines stand where the classes cross on grids of 500 to 10,000 buses.  A
+// Newton solve of five updates, us, class 1 / 3: FP32 factors 1,000 buses
+// x 1,056 (887k fronts x systems) 1,662 / 1,795, x 1,536 (1,290k) 2,153 / 2,052;
+// 1,500 x 704 (887k) 1,865 / 1,858; 2,000 x 480 (802k) 1,900 / 2,086, x 768
+// (1,290k) 2,449 / 2,333; 10,000 x 160 (1,344k, but only 160 systems)
+// 3,075 / 3,280, x 192 3,509 / 3,463.  FP64 2,000 x 416 (699k) 2,371 / 2,226,
+// x 288 (484k) 1,975 / 2,059; 1,000 x 832 (699k) 1,920 / 2,123, x 1,536 3,006 /
+// 2,932.  Class 2 is ahead only on trees of a few hundred fronts: 500 buses (420
+// fronts) x 1,664 (699k) 1,407 / 1,472 and 1,394 in class 2, FP64 1,784 / 1,862
+// and 1,724, x 1,184 (497k) 1,510 / 1,623 and 1,507; 700 buses (589) x 1,184 (696k) 1,509 / 1,640 and 1,780.
+int task_class(int fronts, int batch, int elem_bytes) {
   if (batch == 1) return 0;
   const double work = (double)fronts * batch;
-  return work > 800e3 && batch > 256 ? 3 : work > 200e3 && batch > 128 ? 2 : 1;
+  if (fronts < 550) return work > 1100e3 ? 3 : work > 550e3 ? 2 : 1;
+  return work > (elem_bytes == 8 ? 720e3 : 900e3) && batch > 160 ? 3 : 1;
 }
 
-// Arena caps keep the launch within shared memory (227 KB): elements x
-// lanes x pack x element size per team, programs of at most 44 KB beside it.
+// Solve and transpose solve, us, class 0 / 3: FP32 700 buses x 2,208 (1,298k)
+// 647 / 635, x 2,560 (1,505k) 697 / 664; 1,500 x 1,184 (1,492k) 727 / 727; 2,000 x 544
+// (914k) 599 / 657, x 896 (1,505k) 738 / 765, x 1,792 (3,011k) 1,189 / 1,089; FP64 500 x 2,144
+// (900k) 575 / 627, x 2,624 (1,102k) 753 / 677; 1,000 x 1,312 (1,102k) 769 / 770;
+// 2,000 x 544 749 / 813, x 896 1,056 / 1,032.
+int sweep_class(int fronts, int batch, int elem_bytes) {
+  return (double)fronts * batch > (elem_bytes == 8 ? 1000e3 : 1400e3) && batch > 256 ? 3 : 0;
+}
+
+// Each row is a stage: the most work of a subtree it takes (0: what is left),
+// the work up to which subtrees share a task, the arena's and the program's
+// limits, and the team.  The cuts are steps of two to four in work, so that a
+// stage ends with about as many teams as the GPU holds; the last one takes the
+// top of the tree with the widest team.  Arena caps of the one-warp stages
+// keep several teams resident on an SM; those of the block teams keep the
+// launch within shared memory (227 KB): elements x lanes x pack x element size
+// per team, programs of at most 44 KB beside it.  The numbers are the fastest
+// tried on 2,000 buses x 1 to 1,024 and 10,000 x 64, and nothing finer is
+// claimed for them; which class a batch takes is task_class's choice.
 std::vector<TaskStageSpec> factor_task_specs(int cls, int elem_bytes) {
   const bool d = elem_bytes == 8;
   const int w = 4000, W = 11000;
@@ -557,7 +586,7 @@ std::vector<TaskStageSpec> factor_task_specs(int cls, int elem_bytes) {
 // takes wider groups of scenarios per team and joined subtrees.
 std::vector<TaskStageSpec> sweep_task_specs(int cls) {
   // cut, merge, arena, words, factor elements, warps, lanes, pack
-  if (sweep_class(cls) == 3)
+  if (cls == 3)
     return {{400, 1200, 60, 4000, 80, 1, 16, 1}, {1500, 1500, 160, 4000, 150, 1, 16, 1},
             {0, 0, 2400, 11000, 640, 2, 8, 1}};
   return {{500, 0, 160, 4000, 150, 1, 8, 1}, {2500, 0, 2400, 11000, 640, 2, 8, 1}, {0, 0, 2400, 11000, 640, 2, 8, 1}};
@@ -600,7 +629,7 @@ bool sweep_tasks_pay(const SweepPlan& sp, int fronts, int levels, int batch, int
   if (fronts < kSweepTaskFronts || sp.stages.empty()) return false;
   if (fronts >= 2500) return true;
   const double items = (double)fronts * std::max(batch, 32);
-  if (items > 800e3) return true;  // (much work, whose stages are cut otherwise)
+  if (items > 800e3) return true;
   return sp.chain <= 6.4 * levels - 45 + items / (elem_bytes == 8 ? 30e3 : 45e3);
 }
 

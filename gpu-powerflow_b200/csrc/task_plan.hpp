@@ -60,9 +60,10 @@ constexpr int kTaskFronts = 300;       // smallest trees that factor (sweep) as 
 constexpr int kSweepTaskFronts = 400;
 
 // Classes of batches with stages of their own: 0 a single system; by the
-// fronts x systems of a batch, 1 little, 2 medium, 3 much work.
-int task_class(int fronts, int batch);
-constexpr int sweep_class(int cls) { return cls == 3 ? 3 : 0; }  // classes with the same sweep stages
+// fronts x systems of a batch, 1 little and 3 much work, 2 in between on small
+// trees.  The sweeps have stages of their own for class 0 and 3.
+int task_class(int fronts, int batch, int elem_bytes);
+int sweep_class(int fronts, int batch, int elem_bytes);
 // The stages of a class, for 4- or 8-byte factors.
 std::vector<TaskStageSpec> factor_task_specs(int cls, int elem_bytes);
 std::vector<TaskStageSpec> sweep_task_specs(int cls);
