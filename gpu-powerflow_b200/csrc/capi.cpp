@@ -342,7 +342,12 @@ cls_status cls_singular_flags(cls_handle h, int32_t* out_host, int32_t batch) {
 
 cls_status cls_plan_array(cls_handle h, const char* name, int32_t* out, int64_t capacity, int64_t* len) {
   if (!h || !h->eng) return CLS_INVALID_STATE;
-  return copy_plan_array(*h->eng, name, out, capacity, len) ? CLS_SUCCESS : CLS_INVALID_VALUE;
+  try {
+    return copy_plan_array(*h->eng, name, out, capacity, len) ? CLS_SUCCESS : CLS_INVALID_VALUE;
+  } catch (const std::exception& e) {  // (the task plans are built for the call)
+    h->err = e.what();
+    return CLS_ALLOCATION_FAILED;
+  }
 }
 
 cls_status cls_dump_fronts_csv(cls_handle h, const char* path) {
@@ -743,11 +748,14 @@ pf_status pf_info(pf_handle h, pf_info_t* out) {
 
 pf_status pf_plan_array(pf_handle h, const char* name, int32_t* out, int64_t capacity, int64_t* len) {
   if (!h || !h->eng || h->eng->dim() <= 0) return PF_INVALID_ARGUMENT;
-  if (!copy_plan_array(*h->eng, name, out, capacity, len)) {
+  try {
+    if (copy_plan_array(*h->eng, name, out, capacity, len)) return PF_OK;
     h->err = std::string("unknown plan array or capacity too small: ") + (name ? name : "");
     return PF_INVALID_ARGUMENT;
+  } catch (const std::exception& e) {  // (the task plans are built for the call)
+    h->err = e.what();
+    return PF_RUNTIME_ERROR;
   }
-  return PF_OK;
 }
 
 pf_status pf_dump_fronts_csv(pf_handle h, const char* path) {
