@@ -1126,7 +1126,7 @@ __global__ void __launch_bounds__(256)
 // entries are summed in list order into ts[row * 32] (ts: this lane's column
 // of the block's [fs][32] area in shared memory; rows without entries get 0).
 //
-// single: a batch of one; every lane reads column 0 of the factors, the only
+// SINGLE: a batch of one; every lane reads column 0 of the factors, the only
 // one its tasks write (backward_front).
 // ---------------------------------------------------------------------------
 template <typename T>
@@ -1191,9 +1191,9 @@ __device__ __forceinline__ SweepItem sweep_item(const DevPlan& pl, int level_beg
 // its children's update vectors (extend-add of sum_m L21[.][m] y_m), solves its
 // unit-lower pivot block and emits its own update vector.
 // Shared memory: [fs_cap][32] gathered rows, [8][32] pivot values.
-template <typename T, int NCMAX>
+template <typename T, int NCMAX, bool SINGLE>
 __global__ void __launch_bounds__(256)
-    k_l_forward_level(DevPlan pl, int level_begin, int groups, int Bp, int single, int fs_cap, const T* __restrict__ U,
+    k_l_forward_level(DevPlan pl, int level_begin, int groups, int Bp, int fs_cap, const T* __restrict__ U,
                       const T* __restrict__ L, const double* __restrict__ G, T* __restrict__ TV,
                       T* __restrict__ Yo) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1201,7 +1201,7 @@ __global__ void __launch_bounds__(256)
   const int W = blockDim.x >> 5, warp = threadIdx.x >> 5;
   const SweepItem it = sweep_item(pl, level_begin, groups);
   const int fs = it.fs, nc = it.nc;
-  const size_t b = it.b, fb = single ? 0 : b;
+  const size_t b = it.b, fb = SINGLE ? 0 : b;
   const long long uo = pl.u_off[it.p], lo = pl.l_off[it.p], to = pl.tv_off[it.p];
   T* ts = reinterpret_cast<T*>(smem_raw) + (threadIdx.x & 31);
   T* ys = ts + (size_t)fs_cap * kWarp;
@@ -1244,16 +1244,16 @@ __global__ void __launch_bounds__(256)
 // sum_m U12[m][.] w_m), solves its pivots and emits its own t for the parent.
 // Shared memory: [fs_cap][32] gathered rows, [8][32] pivot values.
 // ---------------------------------------------------------------------------
-template <typename T, int NCMAX>
+template <typename T, int NCMAX, bool SINGLE>
 __global__ void __launch_bounds__(256)
-    k_ut_forward_level(DevPlan pl, int level_begin, int groups, int Bp, int single, int fs_cap, const T* __restrict__ U,
+    k_ut_forward_level(DevPlan pl, int level_begin, int groups, int Bp, int fs_cap, const T* __restrict__ U,
                        const double* __restrict__ G, T* __restrict__ TV, T* __restrict__ Wv) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   chain_allow_next();
   const int W = blockDim.x >> 5, warp = threadIdx.x >> 5;
   const SweepItem it = sweep_item(pl, level_begin, groups);
   const int fs = it.fs, nc = it.nc;
-  const size_t b = it.b, fb = single ? 0 : b;
+  const size_t b = it.b, fb = SINGLE ? 0 : b;
   const long long uo = pl.u_off[it.p], to = pl.tv_off[it.p];
   T* ts = reinterpret_cast<T*>(smem_raw) + (threadIdx.x & 31);
   T* wsm = ts + (size_t)fs_cap * kWarp;
@@ -1294,16 +1294,16 @@ __global__ void __launch_bounds__(256)
 // The warps split the non-pivot rows jj (ancestors' z, from earlier launches)
 // and each sums its rows' L21 terms for every k; warp 0 then solves the pivot
 // block with those partial sums (shared memory [W][8][32]).
-template <typename T, int NCMAX>
+template <typename T, int NCMAX, bool SINGLE>
 __global__ void __launch_bounds__(256)
-    k_lt_backward_level(DevPlan pl, int level_begin, int groups, int Bp, int single, const T* __restrict__ U,
+    k_lt_backward_level(DevPlan pl, int level_begin, int groups, int Bp, const T* __restrict__ U,
                         const T* __restrict__ L, const T* __restrict__ Wv, T* __restrict__ Z) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   chain_allow_next();
   const int W = blockDim.x >> 5, warp = threadIdx.x >> 5;
   const SweepItem it = sweep_item(pl, level_begin, groups);
   const int fs = it.fs, nc = it.nc;
-  const size_t b = it.b, fb = single ? 0 : b;
+  const size_t b = it.b, fb = SINGLE ? 0 : b;
   const long long uo = pl.u_off[it.p], lo = pl.l_off[it.p];
   T* ps = reinterpret_cast<T*>(smem_raw) + (threadIdx.x & 31);
   chain_wait_previous();
@@ -1528,8 +1528,9 @@ void launch_backward_level(const LevelLaunch& lv, const SweepArgs<T>& a, cudaStr
   const long items = (long)lv.count * a.groups;
   if (per_warp > kSmemLimit) {  // U rows too large to stage: read them from global memory
     const int w = lv.bw_wpb > 0 ? lv.bw_wpb : 4;
-    launch_chained(a.single ? k_backward_level<T, false, true> : k_backward_level<T, false, false>, dim3((unsigned)((items + w - 1) / w)), dim3(w * kWarp), 0, s,
-                   "backward sweep", a.plan, lv.begin, lv.count, a.groups, a.Bp, warp_elems, a.U, a.Y, a.X);
+    auto kern = a.single ? k_backward_level<T, false, true> : k_backward_level<T, false, false>;
+    launch_chained(kern, dim3((unsigned)((items + w - 1) / w)), dim3(w * kWarp), 0, s, "backward sweep", a.plan,
+                   lv.begin, lv.count, a.groups, a.Bp, warp_elems, a.U, a.Y, a.X);
     return;
   }
   int wpb = (int)std::min<size_t>(8, kSmemLimit / per_warp);
@@ -1555,8 +1556,9 @@ void launch_backward_top(const LevelLaunch& top, const int* lv_bounds, int nlev,
   const size_t per_warp = (size_t)warp_elems * kWarp * sizeof(T);
   if (per_warp > kSmemLimit) {  // U rows too large to stage: read them from global memory
     const int w = top.bw_wpb > 0 ? top.bw_wpb : 4;
-    launch_chained(a.single ? k_backward_top<T, false, true> : k_backward_top<T, false, false>, dim3((unsigned)a.groups), dim3(w * kWarp), 0, s,
-                   "backward sweep (tree top)", a.plan, lv_bounds, nlev, a.Bp, warp_elems, a.U, a.Y, a.X);
+    auto kern = a.single ? k_backward_top<T, false, true> : k_backward_top<T, false, false>;
+    launch_chained(kern, dim3((unsigned)a.groups), dim3(w * kWarp), 0, s, "backward sweep (tree top)", a.plan,
+                   lv_bounds, nlev, a.Bp, warp_elems, a.U, a.Y, a.X);
     return;
   }
   const int cap = (int)std::min<size_t>(8, kSmemLimit / per_warp);
@@ -1572,8 +1574,9 @@ void launch_ut_forward_level(const LevelLaunch& lv, const AdjointSweepArgs<T>& a
   if (lv.count == 0) return;
   if (lv.max_nc > 8) throw std::runtime_error("panels wider than 8 columns are not supported (max_panel_width <= 8)");
   const long items = (long)lv.count * a.groups;
-  launch_sweep(k_ut_forward_level<T, 8>, items, sweep_warps(items), (size_t)(lv.max_fsz + 8) * kWarp * sizeof(T), s,
-               "adjoint sweep (U^T)", a.plan, lv.begin, a.groups, a.Bp, a.single, lv.max_fsz, a.U, a.G, a.TV, a.W);
+  auto kern = a.single ? k_ut_forward_level<T, 8, true> : k_ut_forward_level<T, 8, false>;
+  launch_sweep(kern, items, sweep_warps(items), (size_t)(lv.max_fsz + 8) * kWarp * sizeof(T), s,
+               "adjoint sweep (U^T)", a.plan, lv.begin, a.groups, a.Bp, lv.max_fsz, a.U, a.G, a.TV, a.W);
 }
 
 template <typename T>
@@ -1581,8 +1584,9 @@ void launch_l_forward_level(const LevelLaunch& lv, const AdjointSweepArgs<T>& a,
   if (lv.count == 0) return;
   if (lv.max_nc > 8) throw std::runtime_error("panels wider than 8 columns are not supported (max_panel_width <= 8)");
   const long items = (long)lv.count * a.groups;
-  launch_sweep(k_l_forward_level<T, 8>, items, sweep_warps(items), (size_t)(lv.max_fsz + 8) * kWarp * sizeof(T), s,
-               "forward substitution", a.plan, lv.begin, a.groups, a.Bp, a.single, lv.max_fsz, a.U, a.L, a.G, a.TV, a.W);
+  auto kern = a.single ? k_l_forward_level<T, 8, true> : k_l_forward_level<T, 8, false>;
+  launch_sweep(kern, items, sweep_warps(items), (size_t)(lv.max_fsz + 8) * kWarp * sizeof(T), s,
+               "forward substitution", a.plan, lv.begin, a.groups, a.Bp, lv.max_fsz, a.U, a.L, a.G, a.TV, a.W);
 }
 
 template <typename T>
@@ -1591,8 +1595,9 @@ void launch_lt_backward_level(const LevelLaunch& lv, const AdjointSweepArgs<T>& 
   if (lv.max_nc > 8) throw std::runtime_error("panels wider than 8 columns are not supported (max_panel_width <= 8)");
   const long items = (long)lv.count * a.groups;
   const int warps = sweep_warps(items);
-  launch_sweep(k_lt_backward_level<T, 8>, items, warps, (size_t)warps * 8 * kWarp * sizeof(T), s,
-               "adjoint sweep (L^T)", a.plan, lv.begin, a.groups, a.Bp, a.single, a.U, a.L, a.W, a.Z);
+  auto kern = a.single ? k_lt_backward_level<T, 8, true> : k_lt_backward_level<T, 8, false>;
+  launch_sweep(kern, items, warps, (size_t)warps * 8 * kWarp * sizeof(T), s,
+               "adjoint sweep (L^T)", a.plan, lv.begin, a.groups, a.Bp, a.U, a.L, a.W, a.Z);
 }
 
 }  // namespace cupf_b200

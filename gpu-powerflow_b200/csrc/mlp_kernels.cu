@@ -789,7 +789,8 @@ int mlp_col_sum_bf16(const void* g, int rows, int cols, float* out, void* stream
 int mlp_col_sum_bf16_parts(const void* g, int rows, int cols, float* out, const double* parts, int n_parts, float* acc,
                            void* stream) {
   return guarded([&] {
-    if (!parts || n_parts < 0 || !acc) throw std::invalid_argument("mlp_col_sum_bf16_parts: parts and acc must not be null");
+    if (!parts || n_parts < 0 || !acc)
+      throw std::invalid_argument("mlp_col_sum_bf16_parts: parts and acc must not be null");
     k_col_sum_bf16<<<(cols + 31) / 32 + 1, dim3(32, 32), 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const __nv_bfloat16*>(g), rows, cols, out, parts, n_parts, acc);
   });
