@@ -111,7 +111,8 @@ def test_autotuner_times_the_launches_that_factor(buses, wide, policy):
         S = torch.tensor(g.scenarios(batch, seed=9), device="cuda")
         V0 = torch.tensor(g.flat_start(batch), device="cuda")
         cfg = cupf.NRConfig(tolerance=1e-8, max_iter=12)
-        assert torch.equal(base.solve_batch_device(S, V0, config=cfg)[0], tuned.solve_batch_device(S, V0, config=cfg)[0])
+        a, b = (h.solve_batch_device(S, V0, config=cfg)[0] for h in (base, tuned))
+        assert torch.equal(a, b)
         n = tuned.plan_array("factor_rest_warps" if wide else "factor_level_warps").size
         assert n > 0 and tuned.plan_array("factor_tuned_launches").tolist() == ([n, 0] if wide else [0, n])
         assert (tuned.plan_array("task_class")[0] >= 0) == bool(wide)
@@ -287,7 +288,8 @@ def test_tasks_solve_like_the_general_kernels(precision, buses, batch, cls):
             assert float((y - b).norm() / b.norm()) <= 300 * eps
 
 
-@pytest.mark.parametrize("buses,batch,cls", [(2000, 1, 0), (2000, 31, 1), (2000, 161, 1), (2000, 540, 3), (500, 1500, 2)])
+@pytest.mark.parametrize("buses,batch,cls", [(2000, 1, 0), (2000, 31, 1), (2000, 161, 1), (2000, 540, 3),
+                                             (500, 1500, 2)])
 @pytest.mark.parametrize("policy", ["FP64", "Mixed", "FP32"])
 def test_newton_and_gradients_of_every_class_keep_the_general_kernels_bits(policy, buses, batch, cls):
     """Two Newton updates, and the gradients at the state they reach, against
@@ -339,3 +341,46 @@ def test_small_trees_take_the_faster_schedule_with_the_same_bits(buses, batch, f
             assert (ls.plan_array("task_class")[0] >= 0) == factor and ls.plan_array("task_sweeps")[0] == sweep
         out.append((ls.solve(b), ls.solve_transpose(b)))
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("batch", [1, 33, 1700])  # the classes' team shapes
+@pytest.mark.parametrize("width", [8, 3])
+@pytest.mark.parametrize("precision", [cupf.CustomPrecision.FP64, cupf.CustomPrecision.FP32])
+def test_fronts_of_every_size_factor_and_solve(precision, width, batch):
+    """Dense diagonally dominant blocks of 1 to 66 rows: fronts of every size a
+    task takes, with every number of pivots, and those beside the tasks; the
+    general kernels' bits, and residuals to the rounding of an LU of such
+    blocks."""
+    import scipy.sparse as sp
+    import torch
+
+    rng = np.random.default_rng(width)
+    sizes = list(range(1, 67)) * (2 if width == 8 else 1)
+    A = sp.block_diag([sp.coo_array(np.ones((n, n))) for n in sizes]).tocsr()
+    A.sort_indices()
+    n = A.shape[0]
+    rp, ci = A.indptr.astype(np.int32), A.indices.astype(np.int32)
+    dtype = torch.float64 if precision == cupf.CustomPrecision.FP64 else torch.float32
+    rows = np.repeat(np.arange(n), np.diff(rp))
+    gen = torch.Generator(device="cuda").manual_seed(batch)
+    vals = torch.randn(batch, ci.size, device="cuda", generator=gen, dtype=dtype)
+    vals[:, torch.tensor(rows == ci, device="cuda")] += 40.0
+    b = torch.tensor(rng.standard_normal((batch, n)), device="cuda")
+    out = []
+    for wide in (0, 1):
+        ls = cupf.LinearSolver(cupf.SolverConfig(precision=int(precision), serial_nd=True, max_panel_width=width,
+                                                 wide_min_front=wide, autotune=False))
+        ls.set_data(rp, ci)
+        ls.analyze()
+        ls.setup(batch)
+        ls.factorize(vals)
+        assert not ls.singular_flags().any()
+        out.append((ls.solve(b), ls.solve_transpose(b)))
+        del ls
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+    # unpivoted LU of diagonally dominant blocks: growth below 2, so the backward
+    # error is at most a few times the rows of a block x the unit roundoff
+    r, c = torch.tensor(rows, device="cuda"), torch.tensor(ci.astype(np.int64), device="cuda")
+    for x, i, j in ((out[0][0][:4], r, c), (out[0][1][:4], c, r)):
+        y = torch.zeros_like(b[:4]).index_add_(1, i, vals[:4].double() * x.double()[:, j])
+        assert float((y - b[:4]).norm() / b[:4].norm()) <= 4 * 66 * torch.finfo(dtype).eps
