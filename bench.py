@@ -53,11 +53,10 @@ MAX_ITER = 10
 
 
 # DRAM traffic (read + write) of one Mixed factorization of the 2,000-bus
-# grid, per 1,024 scenarios: a launch per level, captured with ncu at 256
-# scenarios (72.2 MB read; the writes stay in L2 at that size), scaled by 4
-# (the read traffic grows with the batch; a capture at 1,024 scenarios read
-# 278.8 MB and wrote 11.9 MB)
-FACTOR_DRAM_BYTES_B1024 = 288_800_000
+# grid x 1,024 by its five task launches (k_factor_tasks): 206.2 MB read and
+# 82.1 MB written, one ncu capture with the caches flushed before each launch;
+# scaled by the batch
+FACTOR_DRAM_BYTES_B1024 = 288_300_000
 
 def _peaks() -> dict:
     p = ROOT / "MEASURED_PEAKS.json"
@@ -545,10 +544,9 @@ def run_engine(args) -> None:
     fbytes = factor_bytes_per_scenario(prof, 4) * B
     peaks = _peaks()
     achieved = fbytes / (per_fact_ms / 1e3) / 1e9
-    # DRAM bytes (read + write) of the level launches of one Mixed
-    # factorization at 1,024 scenarios, from one ncu capture of this
-    # workload; scaled by the batch
-    traffic = int(FACTOR_DRAM_BYTES_B1024 * B / 1024) if g.n_bus == 2000 else None
+    # the capture's, where the batch runs the captured stages
+    tasks3 = prof.plan_array("task_class")[0] == 3
+    traffic = int(FACTOR_DRAM_BYTES_B1024 * B / 1024) if g.n_bus == 2000 and tasks3 else None
 
     extras = run_extras(args, dev) if (rank == 0 and world == 1 and not args.no_extra) else None
 

@@ -9,10 +9,12 @@
 // shared memory.  Teams, lanes and workers as in kernels_task.cuh.  The backward
 // sweep U x = y stays with the level kernels: its order makes a front one
 // serial chain, which gains nothing from a team (10,000 buses x 64: 227 us as
-// tasks, 162 us by levels).  Measured: factorize + solve + transpose solve of
-// 1,024 FP32 Jacobians of the 2,000-bus grid 1,744 -> 1,239 us (factorization
-// included), forward and backward through torch on 10,000 buses x 64 9.06 ->
-// 5.26 ms.
+// tasks, 162 us by levels).  Measured, the factorization's tasks included:
+// factorize + solve + transpose solve of 1,024 FP32 Jacobians of the 2,000-bus
+// grid 1,740 -> 1,238 us; forward and backward through torch on 10,000 buses x
+// 64 9.14 -> 5.28 ms.  The stages of one L sweep there
+// (2,000 x 1,024 FP32): 15, 4 and 2 resident warps on an SM, 52, 20 and 13 % of
+// the issue slots, DRAM at 12, 6 and 2 %: the chain of fronts, not bandwidth.
 #pragma once
 
 #include <type_traits>

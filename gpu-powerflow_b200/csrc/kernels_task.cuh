@@ -12,11 +12,12 @@
 // the 32 / LS groups of a warp ("workers") share out a front's elements, so
 // small batches still use every lane of a warp.
 //
-// What bounds it: instruction issue and latency, not memory (FP32, 2,000 buses
-// x 1,024: 30 % of issue slots used at 8 to 16 resident warps, which the
-// arenas' shared memory limits; DRAM below 15 %), hence several scenarios per
-// lane, unrolled small fronts, and joined subtrees that fill the pipeline
-// once per block instead of once per subtree (first stage 101 -> 58 us).
+// What bounds it: instruction issue and latency, not memory (2,000 buses
+// x 1,024 FP32, first stage to last: 11, 12, 7, 5 and 8 resident warps on an SM,
+// which the arenas' shared memory and the registers limit; 47, 47, 28, 29 and
+// 32 % of issue slots used; DRAM at 27, 14, 6, 3 and 2 %), hence several
+// scenarios per lane, unrolled small fronts, and joined subtrees that fill the
+// pipeline once per block instead of once per subtree (first stage 101 -> 58 us).
 // Measured per factorization, level launches -> tasks: 2,000 buses x 1,024
 // FP32 521 -> 293 us and FP64 760 -> 488 us, 10,000 x 64 FP32 540 -> 209 us,
 // 2,000 x 1 140 -> 105 us.

@@ -325,9 +325,10 @@ def test_dense_systems_factor_and_solve(n, precision, tol):
 @pytest.mark.parametrize("batch", [1, 2, 31, 32, 33, 130, 500])
 @pytest.mark.parametrize("policy", ["FP64", "Mixed", "FP32"])
 def test_tasks_give_the_level_kernels_factors(batch, policy):
-    """Solves with the task stages of each batch class against the level
-    launches (wide_min_front = 1 leaves every front to them): the factors are
-    the same bits, and so are the voltages of the first update."""
+    """Solves of a 420-front grid on its schedule (the tree launch for one system,
+    class 1's tasks for more) against the any-size tier (wide_min_front = 1
+    leaves every front to it): the factors are the same bits, and so are the
+    voltages of the first updates.  test_gpu_task_stages.py has every class."""
     import torch
 
     g = G.grid_500()
